@@ -45,6 +45,51 @@ uint32_t pack_nrgba_host(const double c[4]) {
     return out;
 }
 
+// Whether cert_shade's preconditions hold for a draw, and its parameters: the
+// plain form of PhongShader with a constant object colour that can be neither
+// Discard nor blended, non-negative finite light terms and an integer power.
+namespace {
+void fill_cert(const StateView& sv, const ShaderView& shv, CertParams& C) {
+    memset(&C, 0, sizeof(C));
+    if (sv.precision != FGC_PRECISION_PLAIN || shv.kind != FGC_SHADER_PHONG || shv.has_texture ||
+        shv.object_is_discard)
+        return;
+    const double alpha = shv.color[3];
+    if (!(alpha > 0 && alpha <= 1e6) || (sv.alpha_blend && alpha < 1)) return;
+    if (shv.pow_yi < 2 || shv.pow_yi > (uint64_t)kCertPowerMax) return;
+    const double big = 1e6;  // products of the terms stay far inside FP32
+    double l2 = 0, emax = 0;
+    for (int k = 0; k < 3; k++) {
+        const double nonneg[4] = {shv.color[k], shv.ambient[k], shv.diffuse[k], shv.specular[k]};
+        for (double v : nonneg)
+            if (!(v >= 0 && v <= big) || (v > 0 && v < 1e-12)) return;
+        if (!(std::fabs(shv.light[k]) <= big) || !(std::fabs(shv.eye[k]) <= big)) return;
+        l2 += shv.light[k] * shv.light[k];
+        emax = std::max(emax, std::fabs(shv.eye[k]));
+    }
+    if (!(l2 >= 1e-6)) return;
+    C.on = 1;
+    C.power = (int32_t)shv.pow_yi;
+    C.powtol = (float)((C.power + 8) * 1.05 * kCertU);
+    C.ln = (float)(std::sqrt(l2) * 1.0001);
+    C.emax = (float)(emax * 1.0001);
+    double unlit[4];
+    for (int k = 0; k < 3; k++) {
+        C.light[k] = (float)shv.light[k];
+        C.eye[k] = (float)shv.eye[k];
+        C.ambient[k] = (float)shv.ambient[k];
+        C.diffuse[k] = (float)shv.diffuse[k];
+        C.specular[k] = (float)shv.specular[k];
+        C.color255[k] = (float)(shv.color[k] * 255.0);
+        // diffuse = 0 leaves the ambient term: Min(colour * ambient, 1)
+        const double c = shv.color[k] * shv.ambient[k];
+        unlit[k] = c < 1 ? c : 1;
+    }
+    unlit[3] = alpha;
+    C.unlit = pack_nrgba_host(unlit);
+}
+}  // namespace
+
 int fill_views(const fgc_state* st, const fgc_shader* sh, StateView& sv, ShaderView& shv) {
     if (sh->kind != FGC_SHADER_SOLID_COLOR && sh->kind != FGC_SHADER_TEXTURE && sh->kind != FGC_SHADER_PHONG)
         return fail(FGC_ERR_UNSUPPORTED_SHADER, "shader kind is not a built-in shader");
@@ -103,6 +148,7 @@ int fill_views(const fgc_state* st, const fgc_shader* sh, StateView& sv, ShaderV
         shv.tex.w = sh->texture->w;
         shv.tex.h = sh->texture->h;
     }
+    fill_cert(sv, shv, shv.cert);
     return FGC_OK;
 }
 

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/fauxglcuda.h"
+#include "fgc_certshade.cuh"
 #include "fgc_intconv.cuh"
 
 namespace fgc {
@@ -137,6 +138,9 @@ struct ShaderView {
     float eye32[3];
     float ambient32[4], diffuse32[4], specular32[4];
     float power32;
+    // plain-form Phong fragments whose bytes FP32 interval arithmetic can
+    // decide (off: every fragment is shaded in FP64)
+    CertParams cert;
 };
 
 struct StateView {

@@ -223,6 +223,7 @@ struct PassScratch {
     DevBuf<unsigned long long> tiles;
     DevBuf<unsigned char> table;   // item views + lookup starts + per-draw results + counters + status
     DevBuf<double> dbg;
+    DevBuf<PendFrag> pend;         // per raster CTA: fragments awaiting their FP64 colour
     DevBuf<SetupWork> work;        // setup work items (triangles, wireframe edges, lines)
     DevBuf<uint16_t> smeta;        // per element of a setup tile: its setup decision
     DevBuf<uint32_t> cidx;         // per element of a setup tile: its clip_list entry (clipped triangles)

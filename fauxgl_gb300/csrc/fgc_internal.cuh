@@ -227,6 +227,14 @@ struct ScanParams {
 constexpr int32_t kRowTableMinRows = 5;
 __device__ __forceinline__ bool uses_row_table(const PBox& b) { return b.y1 - b.y0 + 1 >= kRowTableMinRows; }
 
+// A fragment that cert_shade could not decide and that passed the depth test:
+// its pixel's colour is formed in FP64 when the band ends or the list fills.
+struct __align__(16) PendFrag {
+    double b0, b1, b2;
+    uint32_t prim;
+    uint32_t pix;
+};
+
 struct RasterParams {
     const ItemView* items;
     ItemStarts starts;
@@ -244,6 +252,8 @@ struct RasterParams {
     int32_t Lmax;               // largest band of the pass (depth staging)
     int32_t win;                // fragment offsets a thread walks per round (wide primitives)
     int32_t su;                 // units a chunk of wide primitives holds
+    PendFrag* pend;             // per CTA pend_cap entries (certified shading), or null
+    uint32_t pend_cap;          // at least F
     const PoolVertex* pool;
     const PoolVertex32* pool32;
     const float4* rf;

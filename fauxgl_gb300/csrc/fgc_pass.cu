@@ -76,6 +76,7 @@ struct PassPlan {
     int precision = FGC_PRECISION_PLAIN;
     int F = 0;
     int su = kSpanUnitsMin;
+    bool cert = false;           // certified shading (some draw of the plain form takes it)
     size_t smem = 0;
     int bin_warps = 1;
     uint32_t scan_tiles = 1;
@@ -230,7 +231,10 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
         v.winner = (c->debug & FGC_DEBUG_WINNER) ? c->winner.p : nullptr;
         v.shaded = (c->debug & FGC_DEBUG_SHADED_COLOR) ? c->shaded.p : nullptr;
         if (v.shaded) P.debug_shaded = true;
+        P.cert = P.cert || v.sh.cert.on;
     }
+    // the FP64 shader output itself is asked for: nothing to certify
+    if (P.debug_shaded) P.cert = false;
     P.vtile[n] = P.vtiles;
     P.stile[n] = P.stiles;
     P.blk[n] = P.nblk;
@@ -244,6 +248,10 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     P.bin_warps = warps;
     return FGC_OK;
 }
+
+// Pending entries per raster CTA (certified shading): a chunk's fragments at
+// least, so that an emptied list holds any chunk.
+uint32_t pend_capacity(int F) { return (uint32_t)std::max(1024, F); }
 
 uint64_t prim_capacity(const PassPlan& P, uint32_t clip_cap) {
     return P.prim_base + (uint64_t)clip_cap * (uint64_t)(6 * P.per_max) + 1;
@@ -361,6 +369,10 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
     }
     FGC_CUDA(S.host_in.ensure(TL.in_bytes() * plans.size()));
     FGC_CUDA(S.host_out.ensure(TL.out_bytes(nmax) * plans.size()));
+    size_t need_pend = 0;
+    for (const PassPlan& P : plans)
+        if (P.cert) need_pend = std::max(need_pend, (size_t)need_grid * pend_capacity(P.F));
+    if (need_pend) FGC_CUDA(S.pend.ensure(need_pend));
     if (need_dbg) {
         size_t most = 0;
         for (const PassPlan& P : plans) most = std::max(most, (size_t)need_grid * P.F * 4);
@@ -613,6 +625,8 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.Lmax = P.Lmax;
         rp.win = std::max(1, std::min(T.window, 256));
         rp.su = P.su;
+        rp.pend = P.cert ? S.pend.p : nullptr;
+        rp.pend_cap = pend_capacity(P.F);
         rp.pool = S.pool.p;
         rp.pool32 = S.pool32.p;
         rp.rf = S.rf.p;
@@ -627,7 +641,7 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         FGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kRasterThreads, P.smem));
         if (per_sm < 1) return fail(FGC_ERR_UNSUPPORTED, "raster kernel does not fit on an SM");
         int rgrid = (int)std::min<uint64_t>((uint64_t)per_sm * D.sms, P.nbands);
-        if (P.debug_shaded) rgrid = std::min<int>(rgrid, (int)need_grid);
+        if (P.debug_shaded || P.cert) rgrid = std::min<int>(rgrid, (int)need_grid);
         FGC_CUDA(launch_raster(P.precision, rgrid, kRasterThreads, P.smem, stream, rp));
         rec.launches++;
         mark(evs, stream);
