@@ -149,6 +149,10 @@ int fill_views(const fgc_state* st, const fgc_shader* sh, StateView& sv, ShaderV
         shv.tex.h = sh->texture->h;
     }
     fill_cert(sv, shv, shv.cert);
+    if (sh->kind == FGC_SHADER_SOLID_COLOR) {
+        shv.solid_nrgba = pack_nrgba_host(shv.color);
+        shv.solid_flags = shv.object_is_discard ? kFragDiscard : (sv.alpha_blend && shv.color[3] < 1) ? kFragBlend : 0;
+    }
     return FGC_OK;
 }
 

@@ -141,6 +141,8 @@ struct ShaderView {
     // plain-form Phong fragments whose bytes FP32 interval arithmetic can
     // decide (off: every fragment is shaded in FP64)
     CertParams cert;
+    uint32_t solid_nrgba;       // SolidColorShader, plain form: NRGBA word
+    uint32_t solid_flags;       // and the raster kernel's Discard / blend flags
 };
 
 struct StateView {

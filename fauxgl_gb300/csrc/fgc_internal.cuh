@@ -229,10 +229,10 @@ __device__ __forceinline__ bool uses_row_table(const PBox& b) { return b.y1 - b.
 
 // A fragment that cert_shade could not decide and that passed the depth test:
 // its pixel's colour is formed in FP64 when the band ends or the list fills.
-struct __align__(16) PendFrag {
-    double b0, b1, b2;
+struct PendFrag {
     uint32_t prim;
-    uint32_t pix;
+    int32_t y;      // its row
+    uint32_t pix;   // its band pixel
 };
 
 struct RasterParams {
@@ -249,6 +249,8 @@ struct RasterParams {
     uint64_t nmat;              // entries of off
     const unsigned long long* pair_total;
     int32_t F;                  // fragment buffer capacity
+    int32_t heads;              // pixel buckets, a power of two
+    int32_t bsize;              // bytes of a fragment's barycentric: 4, or 8 when some draw shades every one in FP64
     int32_t Lmax;               // largest band of the pass (depth staging)
     int32_t win;                // fragment offsets a thread walks per round (wide primitives)
     int32_t su;                 // units a chunk of wide primitives holds
@@ -263,6 +265,12 @@ struct RasterParams {
     unsigned int* status;
     double* dbg;                // debug scratch: gridDim * F * 4 doubles, or null
 };
+
+// Flags of a shaded fragment.
+constexpr uint8_t kFragDiscard = 1;
+constexpr uint8_t kFragBlend = 2;
+constexpr uint8_t kFragPending = 3;  // colour not certified: formed in FP64 if the fragment stays
+constexpr uint8_t kFragBits = 3;     // one of the above or 0; the resolve keeps its ranks in the other bits
 
 // Kernels (grid shapes chosen by the host runtime).
 __global__ void vertex_kernel(VertexParams P);
@@ -302,8 +310,11 @@ __global__ void attrs_kernel(const double* cp, const double* nrm, uint64_t n, AP
 __global__ void f64_to_f32_kernel(const double* in, uint64_t n, float* out);
 __global__ void fp64_rate_kernel(double* out, double a, double b, int iters);
 
-// Pixel buckets of the raster kernel's per-chunk fragment lists.
-constexpr int kRasterHeads = 2048;
+// Pixel buckets of the raster kernel's per-chunk fragment lists: as many as a
+// band has pixels by default, so that only fragments of one pixel share a
+// list; half of that for frames too wide to hold them.
+constexpr int kRasterHeadsMin = 2048;
+constexpr int kRasterHeadsMax = 4096;
 
 // Rows of a band at most.
 constexpr int kBandRowsMax = 128;
@@ -315,28 +326,33 @@ constexpr int kBandRowsMax = 128;
 constexpr int kSpanUnitsMin = 128;
 constexpr int kSpanUnitsMax = 256;
 
+// Pixels of a band at most; a wider frame is refused. The largest band whose
+// depth fits shared memory beside 256 fragments with FP64 barycentrics.
+constexpr int kBandPixelsMax = 26028;
+
 // Bin entries a raster thread examines per chunk, and the chunk's primitive
 // capacity (a chunk of narrow primitives may hold several units per thread).
 constexpr int kChunkPer = 1;
 constexpr int kChunkPrims = 256 * kChunkPer;
 
 // Dynamic shared memory of the raster kernel (layout in fgc_raster.cu), for
-// a fragment buffer of F and su span units: depth[L] f64, fragment
-// b0/b1/b2/z[F] f64, span edge values[su] 3 x f64, scratch 64 u64, fragment
-// key/colour[F] u32, unit slot/row[F] u32, span x/count/offset[su] u32, chunk
-// primitives[kChunkPrims] u32, bucket list heads[kRasterHeads] u16, list
-// links[F] u16, flags[F] u8. The colour buffer is not staged: the band's
-// pixels are read and written in global memory by the CTA that owns them.
-__host__ __device__ inline size_t raster_smem_bytes(int64_t L, int F, int threads, int su) {
+// a fragment buffer of F with barycentrics of bsize bytes and su span units:
+// depth[L] f64, fragment z[F] f64 and b0/b1/b2[F], span edge values[su] 3 x
+// f64, fragment key/colour[F] u32, unit slot/row[256] u32, span
+// x/count/offset[su] u32, chunk primitives[kChunkPrims] u32, bucket list
+// heads[heads] u16, list links[F] u16, flags[F] u8. The colour buffer
+// is not staged: the band's pixels are read and written in global memory by
+// the CTA that owns them.
+__host__ __device__ inline size_t raster_smem_bytes(int64_t L, int F, int threads, int su, int heads, int bsize) {
     size_t b = 0;
     b += (size_t)L * 8;
-    b += (size_t)F * 8 * 4;
+    b += (size_t)F * (8 + 3 * bsize);
     b += (size_t)su * 8 * 3;
-    b += 64 * 8;
-    b += (size_t)F * 4 * 4;
+    b += (size_t)F * 4 * 2;
+    b += (size_t)threads * 4 * 2;
     b += (size_t)su * 4 * 3;
     b += (size_t)(threads > kChunkPrims ? threads : kChunkPrims) * 4;
-    b += (size_t)kRasterHeads * 2;
+    b += (size_t)heads * 2;
     b += (size_t)F * 2;
     b += (size_t)F;
     return (b + 15) & ~(size_t)15;

@@ -76,6 +76,8 @@ struct PassPlan {
     int precision = FGC_PRECISION_PLAIN;
     int F = 0;
     int su = kSpanUnitsMin;
+    int heads = kRasterHeadsMax;
+    int bsize = 4;               // bytes of a fragment's barycentric (8: some draw is shaded in FP64 throughout)
     bool cert = false;           // certified shading (some draw of the plain form takes it)
     size_t smem = 0;
     int bin_warps = 1;
@@ -110,33 +112,38 @@ std::vector<std::vector<uint32_t>> split_passes(const std::vector<PassItem>& ite
     return out;
 }
 
-int fit_fragments(const DevLimits& D, const PassTuning& T, int precision, int32_t Lmax, int& F, int& su,
-                  size_t& smem) {
+int fit_fragments(const DevLimits& D, const PassTuning& T, int precision, int32_t Lmax, int bsize, int& F, int& su,
+                  int& heads, size_t& smem) {
     const int stat = D.raster_static[precision == FGC_PRECISION_MIXED ? 1 : 0];
     const long two_cta = (long)D.smem_per_sm / 2 - D.smem_reserved_per_block - stat;
     const long one_cta = (long)D.smem_per_block_optin - stat;
     F = std::max(256, std::min(T.frag_cap, 4096));
+    heads = kRasterHeadsMax;
     // the larger span arrays first: they also hold the warp queues of the
     // narrow walk, which needs one 32-entry queue per warp (kSpanUnitsMax =
     // the CTA's threads) and is worth more than a larger fragment buffer
     su = kSpanUnitsMax;
-    smem = raster_smem_bytes(Lmax, F, kRasterThreads, su);
+    smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
     // two CTAs per SM (the register budget allows two) when a smaller
     // fragment buffer makes them fit
     while ((long)smem > two_cta && F > 512) {
         F -= 128;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su);
+        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
     }
     while ((long)smem > one_cta && F > 256) {
         F /= 2;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su);
+        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+    }
+    if ((long)smem > one_cta) {
+        heads = kRasterHeadsMin;
+        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
     }
     if ((long)smem > one_cta) {
         // the smaller span arrays (narrow rows then walk thread by thread)
         su = kSpanUnitsMin;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su);
+        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
     }
-    if ((long)smem > one_cta) return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
+    if (Lmax > kBandPixelsMax || (long)smem > one_cta) return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
     return FGC_OK;
 }
 
@@ -235,13 +242,16 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     }
     // the FP64 shader output itself is asked for: nothing to certify
     if (P.debug_shaded) P.cert = false;
+    if (P.precision == FGC_PRECISION_PLAIN)
+        for (const ItemView& v : P.views)
+            if (!(P.cert && v.sh.cert.on) && v.sh.kind != FGC_SHADER_SOLID_COLOR) P.bsize = 8;
     P.vtile[n] = P.vtiles;
     P.stile[n] = P.stiles;
     P.blk[n] = P.nblk;
     P.band[n] = P.nbands;
     if (P.nmat >= 0xFFFFFFFFull) return fail(FGC_ERR_UNSUPPORTED, "pass too large for its bin matrix");
     P.scan_tiles = (uint32_t)ceil_div(P.nmat, 2048);
-    int rc = fit_fragments(D, T, P.precision, P.Lmax, P.F, P.su, P.smem);
+    int rc = fit_fragments(D, T, P.precision, P.Lmax, P.bsize, P.F, P.su, P.heads, P.smem);
     if (rc) return rc;
     const int warps = (int)std::min<int64_t>(8, (96 * 1024) / ((int64_t)P.max_nbands * 4));
     if (warps < 1) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands for binning");
@@ -622,6 +632,8 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.nmat = P.nmat;
         rp.pair_total = &dc->pair_total;
         rp.F = P.F;
+        rp.bsize = P.bsize;
+        rp.heads = P.heads;
         rp.Lmax = P.Lmax;
         rp.win = std::max(1, std::min(T.window, 256));
         rp.su = P.su;
