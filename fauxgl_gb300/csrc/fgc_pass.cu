@@ -157,6 +157,23 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     P.blk.assign(n + 1, 0);
     P.band.assign(n + 1, 0);
     P.precision = sub.items[idx[0]].sv.precision;
+    // Small passes take smaller bands and binning blocks than the tuning
+    // allows, so that every raster CTA (two per SM) has a band and the
+    // binning a block per CTA slot: at 4,096 pixels a 512x512 frame is 64
+    // bands, and its raster stage 225 us; at 862 (one 512-pixel row) 94 us,
+    // 128x128 223 -> 41 us, 1280x720 197 -> 166 us, though primitives meet more
+    // bands. Below that smaller bands no longer pay (1080p at one row a band:
+    // 293 -> 305 us). Binning 81,920 triangles in 20 blocks of 4,096 took 61 us,
+    // in 304 39 us; below 256 primitives a block there is nothing left to gain.
+    uint64_t pass_px = 0, pass_prims = 0;
+    for (uint32_t i : idx) {
+        const PassItem& it = sub.items[i];
+        pass_px += (uint64_t)it.ctx->N;
+        pass_prims += it.tc * (it.sv.wireframe ? 6 : 1) + it.lc * 2;
+    }
+    const int64_t band_pixels = std::min<int64_t>(T.band_pixels, (int64_t)(pass_px / (2 * (uint64_t)D.sms)));
+    const int64_t bin_prims =
+        std::min<int64_t>(T.prims_per_bin_block, std::max<int64_t>(256, (int64_t)(pass_prims / (2 * (uint64_t)D.sms))));
     for (uint32_t j = 0; j < n; j++) {
         const PassItem& it = sub.items[idx[j]];
         const fgc_context* c = it.ctx;
@@ -174,7 +191,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
         v.W = c->W;
         v.H = c->H;
         v.N = c->N;
-        int64_t R = std::max<int64_t>(1, T.band_pixels / c->W);
+        int64_t R = std::max<int64_t>(1, band_pixels / c->W);
         R = std::min<int64_t>(R, kBandRowsMax);
         R = std::min<int64_t>(R, c->H);
         if (R * c->W > 65535) return fail(FGC_ERR_UNSUPPORTED, "frame width above 65535 pixels is not supported");
@@ -184,7 +201,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
         if (v.nbands > (uint32_t)kMaxBands) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands");
         const int per = it.sv.wireframe ? 6 : 1;
         const uint64_t prims = it.tc * per + it.lc * 2;
-        v.nblk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, ceil_div(prims, T.prims_per_bin_block)),
+        v.nblk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, ceil_div(prims, (uint64_t)bin_prims)),
                                               (uint64_t)2 * D.sms);
         const bool draws = it.tc > 0 || it.lc > 0;
         const uint32_t vt = draws ? (uint32_t)ceil_div(it.mesh->nuniq, kVertexTile) : 0;
