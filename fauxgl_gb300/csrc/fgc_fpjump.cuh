@@ -75,6 +75,18 @@ FGC_HD bool fj_mul_fits(uint64_t x, uint64_t y, uint64_t z) {
 #endif
 }
 
+// x / y where the quotient is below 2^20 (x < 2^54, 0 < y < 2^54). The FP32
+// quotient is within one of it -- two rounded operands and a rounded division,
+// 3 * 2^-24 relative -- and two exact products settle it; a 64-bit division is
+// a subroutine of some 100 instructions in the middle of every jump's chain
+// (the close-up frame of 1.55 M pixels: row starts 320 -> 260 us).
+FGC_HD uint64_t fj_div_small(uint64_t x, uint64_t y) {
+    uint64_t c = (uint64_t)((float)x / (float)y);
+    if (c * y > x) c--;
+    if ((c + 1) * y <= x) c++;
+    return c;
+}
+
 // t = s; repeat k times: t = RN(t + a). Returns t.
 FGC_HD double repeat_add(double s, double a, uint64_t k) {
     const uint64_t kSign = 0x8000000000000000ull;
@@ -134,7 +146,7 @@ FGC_HD double repeat_add(double s, double a, uint64_t k) {
         }
         // all k remaining steps usually fit: only a jump that reaches the
         // binade's end needs the division
-        const uint64_t n = fj_mul_fits(k - 1, d, avail) ? k : avail / d + 1;
+        const uint64_t n = fj_mul_fits(k - 1, d, avail) ? k : (k <= (1u << 20) ? fj_div_small(avail, d) : avail / d) + 1;
         m = grow ? m + n * d : m - n * d;
         k -= n;
         s = fj_double((sb & kSign) | ((uint64_t)es << 52) | (m - kHidden));

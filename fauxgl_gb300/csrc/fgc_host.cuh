@@ -186,7 +186,7 @@ struct PassTuning {
     int64_t band_pixels = 4096;         // pixels per band, rounded to whole rows
     int64_t prims_per_bin_block = 4096; // raster primitives per binning block
     int frag_cap = 1024;                // upper bound of the raster fragment buffer
-    int window = 8;                     // raster fragment offsets per thread and round (wide primitives)
+    int window = 8;                     // accepted and reported; the raster stage sizes its runs itself
 };
 
 // One draw of a pass, as the host describes it.

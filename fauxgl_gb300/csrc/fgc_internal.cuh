@@ -252,7 +252,6 @@ struct RasterParams {
     int32_t heads;              // pixel buckets, a power of two
     int32_t bsize;              // bytes of a fragment's barycentric: 4, or 8 when some draw shades every one in FP64
     int32_t Lmax;               // largest band of the pass (depth staging)
-    int32_t win;                // fragment offsets a thread walks per round (wide primitives)
     int32_t su;                 // units a chunk of wide primitives holds
     PendFrag* pend;             // per CTA pend_cap entries (certified shading), or null
     uint32_t pend_cap;          // at least F

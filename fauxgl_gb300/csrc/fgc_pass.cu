@@ -652,7 +652,6 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.bsize = P.bsize;
         rp.heads = P.heads;
         rp.Lmax = P.Lmax;
-        rp.win = std::max(1, std::min(T.window, 256));
         rp.su = P.su;
         rp.pend = P.cert ? S.pend.p : nullptr;
         rp.pend_cap = pend_capacity(P.F);
