@@ -32,6 +32,99 @@ int grid_for(uint64_t n, int block, int cap) {
     return (int)g;
 }
 
+// ---------------------------------------------------------------------------
+// Mesh memory pools and call streams, one set per device
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int kMaxDevices = 64;
+constexpr size_t kKeptStreams = 8;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t free_stream = nullptr;
+    std::vector<cudaStream_t> idle;
+};
+std::mutex g_pool_mu;
+DevicePool g_pools[kMaxDevices];
+
+// The current device's set, created on first use (g_pool_mu held).
+cudaError_t device_pool(DevicePool** out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    DevicePool& P = g_pools[dev];
+    if (!P.pool) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t keep = kPoolKeep;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P.free_stream, cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        P.pool = pool;
+    }
+    *out = &P;
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+    DevicePool* P = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        const cudaError_t e = device_pool(&P);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaMallocFromPoolAsync(p, bytes, P->pool, s);
+}
+
+void pool_free(void* p, cudaStream_t s) { cudaFreeAsync(p, s); }
+
+bool pool_trim() {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    bool any = false;
+    for (DevicePool& P : g_pools)
+        if (P.pool) any = cudaMemPoolTrimTo(P.pool, 0) == cudaSuccess || any;
+    return any;
+}
+
+cudaError_t take_stream(int device, cudaStream_t* s) {
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (device >= 0 && device < kMaxDevices && !g_pools[device].idle.empty()) {
+            *s = g_pools[device].idle.back();
+            g_pools[device].idle.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+
+void give_stream(int device, cudaStream_t s) {
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (device >= 0 && device < kMaxDevices && g_pools[device].idle.size() < kKeptStreams) {
+            g_pools[device].idle.push_back(s);
+            return;
+        }
+    }
+    cudaStreamDestroy(s);
+}
+
+cudaStream_t free_stream() {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool* P = nullptr;
+    return device_pool(&P) == cudaSuccess ? P->free_stream : nullptr;
+}
+
 uint32_t pack_nrgba_host(const double c[4]) {
     uint32_t out = 0;
     for (int k = 0; k < 4; k++) {
@@ -251,10 +344,8 @@ int draw(fgc_context* c, const fgc_mesh* m, uint64_t tf, uint64_t tc, uint64_t l
 // be null: zero normals). Runs on stream s and waits for it.
 int mesh_weld_attrs(fgc_mesh* m, cudaStream_t s, int sms, const double* cp, const double* nrm, uint64_t V) {
     int rc = FGC_OK;
-    DevBuf<uint32_t> table, slot_of, minc, flag, uid;
-    DevBuf<unsigned long long> tiles;
-    DevBuf<unsigned int> st, tick;
-    unsigned long long* h_tot = nullptr;
+    TempBuf<uint32_t> table, slot_of, flag, uid;  // table: hash slots, then each slot's first corner
+    TempBuf<unsigned long long> tiles;            // total, scan tiles, then status and ticket
     auto step = [&](cudaError_t err, const char* what) {
         if (err != cudaSuccess && rc == FGC_OK) rc = fail(FGC_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(err));
         return rc == FGC_OK;
@@ -264,48 +355,44 @@ int mesh_weld_attrs(fgc_mesh* m, cudaStream_t s, int sms, const double* cp, cons
         // weld positions
         uint64_t tsize = 1;
         while (tsize < 2 * V) tsize <<= 1;
-        if (!step(table.ensure(tsize), "alloc weld table")) break;
-        if (!step(minc.ensure(tsize), "alloc weld table")) break;
-        if (!step(slot_of.ensure(V), "alloc weld") || !step(flag.ensure(V), "alloc weld") || !step(uid.ensure(V), "alloc weld")) break;
-        if (!step(st.ensure(1), "alloc status") || !step(cudaMemsetAsync(st.p, 0, 4, s), "zero status")) break;
-        if (!step(cudaMemsetAsync(table.p, 0xFF, tsize * 4, s), "init table")) break;
-        if (!step(cudaMemsetAsync(minc.p, 0xFF, tsize * 4, s), "init table")) break;
-        weld_insert_kernel<<<grid, 256, 0, s>>>(cp, V, table.p, tsize - 1, slot_of.p, minc.p, st.p);
-        weld_flag_kernel<<<grid, 256, 0, s>>>(slot_of.p, minc.p, V, flag.p);
         const uint64_t scan_tiles = (V + 2047) / 2048;
-        if (!step(tiles.ensure(scan_tiles + 2), "alloc scan") || !step(cudaMemsetAsync(tiles.p, 0, (scan_tiles + 2) * 8, s), "zero scan")) break;
+        if (!step(table.ensure(2 * tsize, s), "alloc weld table") || !step(slot_of.ensure(V, s), "alloc weld") ||
+            !step(flag.ensure(V, s), "alloc weld") || !step(uid.ensure(V, s), "alloc weld") ||
+            !step(tiles.ensure(scan_tiles + 2, s), "alloc scan"))
+            break;
+        uint32_t* minc = table.p + tsize;
+        unsigned int* st = (unsigned int*)(tiles.p + scan_tiles + 1);
+        if (!step(cudaMemsetAsync(table.p, 0xFF, 2 * tsize * 4, s), "init table")) break;
+        if (!step(cudaMemsetAsync(tiles.p, 0, (scan_tiles + 2) * 8, s), "zero scan")) break;
+        weld_insert_kernel<<<grid, 256, 0, s>>>(cp, V, table.p, tsize - 1, slot_of.p, minc, st);
+        weld_flag_kernel<<<grid, 256, 0, s>>>(slot_of.p, minc, V, flag.p);
         ScanParams sp;
         sp.n_dev = nullptr;
         sp.in = flag.p;
         sp.out = uid.p;
         sp.n = V;
-        sp.lb = Lookback{tiles.p + 1, (unsigned int*)(st.p), st.p, tiles.p};
-        // the scan's ticket counter and status share the zeroed status word's
-        // neighbour: use a dedicated zeroed word instead
-        if (!step(tick.ensure(1), "alloc ticket") || !step(cudaMemsetAsync(tick.p, 0, 4, s), "zero ticket")) break;
-        sp.lb.ticket = tick.p;
+        sp.lb = Lookback{tiles.p + 1, st + 1, st, tiles.p};
         scan_u32_kernel<<<(unsigned)scan_tiles, 256, 0, s>>>(sp);
         if (!step(cudaGetLastError(), "weld kernels")) break;
-        if (!step(cudaMallocHost((void**)&h_tot, 16), "alloc pinned")) break;
-        if (!step(cudaMemcpyAsync(h_tot, tiles.p, 8, cudaMemcpyDeviceToHost, s), "read unique count")) break;
-        if (!step(cudaMemcpyAsync(h_tot + 1, st.p, 4, cudaMemcpyDeviceToHost, s), "read status")) break;
+        unsigned long long h_tot[2] = {0, 0};
+        if (!step(cudaMemcpyAsync(&h_tot[0], tiles.p, 8, cudaMemcpyDeviceToHost, s), "read unique count")) break;
+        if (!step(cudaMemcpyAsync(&h_tot[1], st, 4, cudaMemcpyDeviceToHost, s), "read status")) break;
         if (!step(cudaStreamSynchronize(s), "weld")) break;
-        if (((unsigned int*)(h_tot + 1))[0] != 0) {
+        if ((unsigned int)h_tot[1] != 0) {
             rc = fail(FGC_ERR_DEVICE_LIMIT, "mesh weld failed");
             break;
         }
         m->nuniq = h_tot[0];
-        if (!step(m->ux.ensure(m->nuniq + 1), "alloc unique") || !step(m->uy.ensure(m->nuniq + 1), "alloc unique") ||
-            !step(m->uz.ensure(m->nuniq + 1), "alloc unique") || !step(m->corner_uniq.ensure(V), "alloc index"))
+        if (!step(m->ux.ensure(m->nuniq + 1, s), "alloc unique") || !step(m->uy.ensure(m->nuniq + 1, s), "alloc unique") ||
+            !step(m->uz.ensure(m->nuniq + 1, s), "alloc unique") || !step(m->corner_uniq.ensure(V, s), "alloc index"))
             break;
-        weld_emit_kernel<<<grid, 256, 0, s>>>(cp, slot_of.p, minc.p, uid.p, V, m->ux.p, m->uy.p, m->uz.p,
+        weld_emit_kernel<<<grid, 256, 0, s>>>(cp, slot_of.p, minc, uid.p, V, m->ux.p, m->uy.p, m->uz.p,
                                               m->corner_uniq.p);
-        if (!step(m->pn64.ensure(V), "alloc attributes") || !step(m->pn32.ensure(V), "alloc attributes")) break;
+        if (!step(m->pn64.ensure(V, s), "alloc attributes") || !step(m->pn32.ensure(V, s), "alloc attributes")) break;
         attrs_kernel<<<grid, 256, 0, s>>>(cp, nrm, V, m->pn64.p, m->pn32.p);
         if (!step(cudaGetLastError(), "attribute kernels")) break;
     } while (0);
     cudaStreamSynchronize(s);
-    if (h_tot) cudaFreeHost(h_tot);
     return rc;
 }
 
@@ -536,13 +623,13 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaStream_t s;
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    cudaError_t e = take_stream(dev, &s);
     if (e != cudaSuccess) {
         delete m;
         return fail(FGC_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
     }
     int rc = FGC_OK;
-    DevBuf<double> cp, nrm;
+    TempBuf<double> cp, nrm;
     auto step = [&](cudaError_t err, const char* what) {
         if (err != cudaSuccess && rc == FGC_OK) rc = fail(FGC_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(err));
         return rc == FGC_OK;
@@ -550,12 +637,12 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
     const int grid = grid_for(V, 256, sms * 16);
     do {
         if (V == 0) break;
-        if (!step(cp.ensure(V * 3), "alloc positions")) break;
+        if (!step(cp.ensure(V * 3, s), "alloc positions")) break;
         if (ntri && !step(cudaMemcpyAsync(cp.p, tri_pos, ntri * 9 * 8, cudaMemcpyHostToDevice, s), "copy positions")) break;
         if (nline && !step(cudaMemcpyAsync(cp.p + ntri * 9, line_pos, nline * 6 * 8, cudaMemcpyHostToDevice, s), "copy positions")) break;
         const bool have_nrm = tri_nrm || line_nrm;
         if (have_nrm) {
-            if (!step(nrm.ensure(V * 3), "alloc normals")) break;
+            if (!step(nrm.ensure(V * 3, s), "alloc normals")) break;
             if (!step(cudaMemsetAsync(nrm.p, 0, V * 3 * 8, s), "zero normals")) break;
             if (tri_nrm && !step(cudaMemcpyAsync(nrm.p, tri_nrm, ntri * 9 * 8, cudaMemcpyHostToDevice, s), "copy normals")) break;
             if (line_nrm && !step(cudaMemcpyAsync(nrm.p + ntri * 9, line_nrm, nline * 6 * 8, cudaMemcpyHostToDevice, s), "copy normals")) break;
@@ -564,7 +651,7 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
         if (rc != FGC_OK) break;
         if (tri_tex || line_tex) {
             m->has_tex = true;
-            if (!step(m->tex64.ensure(V * 2), "alloc texcoords") || !step(m->tex32.ensure(V * 2), "alloc texcoords")) break;
+            if (!step(m->tex64.ensure(V * 2, s), "alloc texcoords") || !step(m->tex32.ensure(V * 2, s), "alloc texcoords")) break;
             if (!step(cudaMemsetAsync(m->tex64.p, 0, V * 2 * 8, s), "zero texcoords")) break;
             if (tri_tex && !step(cudaMemcpyAsync(m->tex64.p, tri_tex, ntri * 6 * 8, cudaMemcpyHostToDevice, s), "copy texcoords")) break;
             if (line_tex && !step(cudaMemcpyAsync(m->tex64.p + ntri * 6, line_tex, nline * 4 * 8, cudaMemcpyHostToDevice, s), "copy texcoords")) break;
@@ -572,7 +659,7 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
         }
         if (tri_col || line_col) {
             m->has_col = true;
-            if (!step(m->col64.ensure(V * 4), "alloc colours") || !step(m->col32.ensure(V * 4), "alloc colours")) break;
+            if (!step(m->col64.ensure(V * 4, s), "alloc colours") || !step(m->col32.ensure(V * 4, s), "alloc colours")) break;
             if (!step(cudaMemsetAsync(m->col64.p, 0, V * 4 * 8, s), "zero colours")) break;
             if (tri_col && !step(cudaMemcpyAsync(m->col64.p, tri_col, ntri * 12 * 8, cudaMemcpyHostToDevice, s), "copy colours")) break;
             if (line_col && !step(cudaMemcpyAsync(m->col64.p + ntri * 12, line_col, nline * 8 * 8, cudaMemcpyHostToDevice, s), "copy colours")) break;
@@ -581,8 +668,10 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
         if (!step(cudaGetLastError(), "attribute kernels")) break;
         step(cudaStreamSynchronize(s), "mesh upload");
     } while (0);
+    cp.release();
+    nrm.release();
     cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
+    give_stream(dev, s);
     if (rc != FGC_OK) {
         delete m;
         return rc;

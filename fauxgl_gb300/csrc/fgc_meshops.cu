@@ -351,13 +351,13 @@ struct Work {
     Work(int device) : dev(device) {
         cudaSetDevice(dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+        cudaError_t e = take_stream(dev, &s);
         if (e != cudaSuccess) rc = fail(FGC_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
     }
     ~Work() {
         if (s) {
             cudaStreamSynchronize(s);
-            cudaStreamDestroy(s);
+            give_stream(dev, s);
         }
     }
     bool ok(cudaError_t e, const char* what) {
@@ -369,10 +369,10 @@ struct Work {
 
 // Exclusive scan of n u32 on the device; *total receives the sum.
 bool scan_u32(Work& W, const uint32_t* in, uint32_t* out, uint64_t n, uint64_t* total) {
-    DevBuf<unsigned long long> tiles;
-    DevBuf<unsigned int> words;  // ticket, status
+    TempBuf<unsigned long long> tiles;
+    TempBuf<unsigned int> words;  // ticket, status
     const uint64_t nt = (n + 2047) / 2048;
-    if (!W.ok(tiles.ensure(nt + 2), "alloc scan") || !W.ok(words.ensure(2), "alloc scan")) return false;
+    if (!W.ok(tiles.ensure(nt + 2, W.s), "alloc scan") || !W.ok(words.ensure(2, W.s), "alloc scan")) return false;
     if (!W.ok(cudaMemsetAsync(tiles.p, 0, (nt + 2) * 8, W.s), "zero scan") ||
         !W.ok(cudaMemsetAsync(words.p, 0, 8, W.s), "zero scan"))
         return false;
@@ -403,35 +403,35 @@ bool scan_u32(Work& W, const uint32_t* in, uint32_t* out, uint64_t n, uint64_t* 
 
 // Groups of the first V corners of a mesh by position (Go map keys).
 struct Groups {
-    DevBuf<uint32_t> gid, start, count, member;
+    TempBuf<uint32_t> gid, start, count, member;
     uint64_t G = 0;  // group slots (some may be empty)
 };
 
 bool build_groups(Work& W, const fgc_mesh* m, uint64_t V, Groups& Gr) {
-    DevBuf<double> key;
-    DevBuf<uint8_t> nanf;
-    DevBuf<uint32_t> table, slot_of, minc, flag, uid, cursor;
-    DevBuf<unsigned int> st;
+    TempBuf<double> key;
+    TempBuf<uint8_t> nanf;
+    TempBuf<uint32_t> table, slot_of, flag, uid, cursor;  // table: hash slots, then each slot's first corner
+    TempBuf<unsigned int> st;
     uint64_t tsize = 1;
     while (tsize < 2 * V) tsize <<= 1;
-    if (!W.ok(key.ensure(3 * V), "alloc keys") || !W.ok(nanf.ensure(V), "alloc keys") ||
-        !W.ok(table.ensure(tsize), "alloc table") || !W.ok(minc.ensure(tsize), "alloc table") ||
-        !W.ok(slot_of.ensure(V), "alloc groups") || !W.ok(flag.ensure(V), "alloc groups") ||
-        !W.ok(uid.ensure(V), "alloc groups") || !W.ok(cursor.ensure(V), "alloc groups") ||
-        !W.ok(Gr.gid.ensure(V), "alloc groups") || !W.ok(Gr.start.ensure(V), "alloc groups") ||
-        !W.ok(Gr.count.ensure(V), "alloc groups") || !W.ok(Gr.member.ensure(V), "alloc groups") ||
-        !W.ok(st.ensure(1), "alloc status"))
+    if (!W.ok(key.ensure(3 * V, W.s), "alloc keys") || !W.ok(nanf.ensure(V, W.s), "alloc keys") ||
+        !W.ok(table.ensure(2 * tsize, W.s), "alloc table") ||
+        !W.ok(slot_of.ensure(V, W.s), "alloc groups") || !W.ok(flag.ensure(V, W.s), "alloc groups") ||
+        !W.ok(uid.ensure(V, W.s), "alloc groups") || !W.ok(cursor.ensure(V, W.s), "alloc groups") ||
+        !W.ok(Gr.gid.ensure(V, W.s), "alloc groups") || !W.ok(Gr.start.ensure(V, W.s), "alloc groups") ||
+        !W.ok(Gr.count.ensure(V, W.s), "alloc groups") || !W.ok(Gr.member.ensure(V, W.s), "alloc groups") ||
+        !W.ok(st.ensure(1, W.s), "alloc status"))
         return false;
     const int grid = W.grid(V);
-    if (!W.ok(cudaMemsetAsync(table.p, 0xFF, tsize * 4, W.s), "init table") ||
-        !W.ok(cudaMemsetAsync(minc.p, 0xFF, tsize * 4, W.s), "init table") ||
+    uint32_t* const minc = table.p + tsize;
+    if (!W.ok(cudaMemsetAsync(table.p, 0xFF, 2 * tsize * 4, W.s), "init table") ||
         !W.ok(cudaMemsetAsync(st.p, 0, 4, W.s), "zero status") ||
         !W.ok(cudaMemsetAsync(Gr.count.p, 0, V * 4, W.s), "zero counts") ||
         !W.ok(cudaMemsetAsync(cursor.p, 0, V * 4, W.s), "zero cursors"))
         return false;
     group_keys_kernel<<<grid, 256, 0, W.s>>>(m->pn64.p, V, key.p, nanf.p);
-    weld_insert_kernel<<<grid, 256, 0, W.s>>>(key.p, V, table.p, tsize - 1, slot_of.p, minc.p, st.p);
-    weld_flag_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc.p, V, flag.p);
+    weld_insert_kernel<<<grid, 256, 0, W.s>>>(key.p, V, table.p, tsize - 1, slot_of.p, minc, st.p);
+    weld_flag_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc, V, flag.p);
     if (!W.ok(cudaGetLastError(), "group kernels")) return false;
     uint64_t nrep = 0;
     if (!scan_u32(W, flag.p, uid.p, V, &nrep)) return false;
@@ -444,7 +444,7 @@ bool build_groups(Work& W, const fgc_mesh* m, uint64_t V, Groups& Gr) {
         return false;
     }
     Gr.G = nrep;
-    group_ids_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc.p, uid.p, nanf.p, V, Gr.gid.p, Gr.count.p);
+    group_ids_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc, uid.p, nanf.p, V, Gr.gid.p, Gr.count.p);
     uint64_t total = 0;
     if (!W.ok(cudaGetLastError(), "group kernels") || !scan_u32(W, Gr.count.p, Gr.start.p, Gr.G, &total)) return false;
     group_fill_kernel<<<grid, 256, 0, W.s>>>(Gr.gid.p, Gr.start.p, cursor.p, V, Gr.member.p);
@@ -457,8 +457,8 @@ bool smooth_normals_into(Work& W, const fgc_mesh* m, double* out) {
     const uint64_t V = 3 * m->ntri;
     Groups Gr;
     if (!build_groups(W, m, V, Gr)) return false;
-    DevBuf<double> gsum;
-    if (!W.ok(gsum.ensure(3 * std::max<uint64_t>(Gr.G, 1)), "alloc sums")) return false;
+    TempBuf<double> gsum;
+    if (!W.ok(gsum.ensure(3 * std::max<uint64_t>(Gr.G, 1), W.s), "alloc sums")) return false;
     smooth_sum_kernel<<<W.grid(Gr.G), 256, 0, W.s>>>(m->pn64.p, Gr.start.p, Gr.count.p, Gr.member.p, Gr.G, gsum.p);
     smooth_assign_kernel<<<W.grid(V), 256, 0, W.s>>>(Gr.gid.p, gsum.p, V, out);
     return W.ok(cudaGetLastError(), "smoothing kernels");
@@ -543,15 +543,15 @@ int fgc_mesh_load_stl(const void* data, uint64_t nbytes, fgc_mesh** out) {
     cudaGetDevice(&dev);
     Work W(dev);
     if (W.rc) return W.rc;
-    DevBuf<double> cp, nrm;
-    DevBuf<uint8_t> rec;
+    TempBuf<double> cp, nrm;
+    TempBuf<uint8_t> rec;
     uint64_t T = 0;
     if (count * 50 + 84 == nbytes) {  // binary (LoadSTL's size test)
         T = count;
         if (3 * T >= 0x7FFFFFFFull) return fail(FGC_ERR_UNSUPPORTED, "mesh has too many corners (2^31 limit)");
         if (T) {
-            if (!W.ok(rec.ensure(50 * T), "alloc records") || !W.ok(cp.ensure(9 * T), "alloc positions") ||
-                !W.ok(nrm.ensure(9 * T), "alloc normals") ||
+            if (!W.ok(rec.ensure(50 * T, W.s), "alloc records") || !W.ok(cp.ensure(9 * T, W.s), "alloc positions") ||
+                !W.ok(nrm.ensure(9 * T, W.s), "alloc normals") ||
                 !W.ok(cudaMemcpyAsync(rec.p, b + 84, 50 * T, cudaMemcpyHostToDevice, W.s), "copy records"))
                 return W.rc;
             stl_decode_kernel<<<W.grid(T), 256, 0, W.s>>>(rec.p, T, cp.p, nrm.p);
@@ -565,7 +565,7 @@ int fgc_mesh_load_stl(const void* data, uint64_t nbytes, fgc_mesh** out) {
         T = nv / 3;
         if (3 * T >= 0x7FFFFFFFull) return fail(FGC_ERR_UNSUPPORTED, "mesh has too many corners (2^31 limit)");
         if (T) {
-            if (!W.ok(cp.ensure(9 * T), "alloc positions") || !W.ok(nrm.ensure(9 * T), "alloc normals") ||
+            if (!W.ok(cp.ensure(9 * T, W.s), "alloc positions") || !W.ok(nrm.ensure(9 * T, W.s), "alloc normals") ||
                 !W.ok(cudaMemcpyAsync(cp.p, pos.data(), 9 * T * 8, cudaMemcpyHostToDevice, W.s), "copy positions"))
                 return W.rc;
             face_normals_kernel<<<W.grid(T), 256, 0, W.s>>>(cp.p, T, nrm.p);
@@ -595,8 +595,8 @@ int fgc_mesh_smooth_normals_threshold(fgc_mesh* m, double radians) {
     if (W.rc) return W.rc;
     const double threshold = std::cos(radians);
     Groups Gr;
-    DevBuf<double> out;
-    if (!build_groups(W, m, V, Gr) || !W.ok(out.ensure(3 * V), "alloc normals")) return W.rc;
+    TempBuf<double> out;
+    if (!build_groups(W, m, V, Gr) || !W.ok(out.ensure(3 * V, W.s), "alloc normals")) return W.rc;
     smooth_threshold_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, V,
                                                          threshold, out.p);
     set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, V, m->pn64.p, m->pn32.p);
@@ -611,8 +611,8 @@ int fgc_mesh_smooth_normals(fgc_mesh* m) {
     if (V == 0) return FGC_OK;
     Work W(m->device);
     if (W.rc) return W.rc;
-    DevBuf<double> out;
-    if (!W.ok(out.ensure(3 * V), "alloc normals") || !smooth_normals_into(W, m, out.p)) return W.rc;
+    TempBuf<double> out;
+    if (!W.ok(out.ensure(3 * V, W.s), "alloc normals") || !smooth_normals_into(W, m, out.p)) return W.rc;
     set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, V, m->pn64.p, m->pn32.p);
     W.ok(cudaGetLastError(), "smoothing kernels");
     W.ok(cudaStreamSynchronize(W.s), "smoothing");
@@ -628,15 +628,15 @@ int fgc_mesh_sharp_edges(const fgc_mesh* m, double angle_threshold, fgc_mesh** o
     const uint64_t T = m->ntri, E = 3 * T;
     if (T == 0) return line_mesh(W, nullptr, 0, out);
     Groups Gr;
-    DevBuf<uint32_t> flag, pos;
-    DevBuf<double> lines;
-    if (!build_groups(W, m, 3 * T, Gr) || !W.ok(flag.ensure(E), "alloc flags") || !W.ok(pos.ensure(E), "alloc flags"))
+    TempBuf<uint32_t> flag, pos;
+    TempBuf<double> lines;
+    if (!build_groups(W, m, 3 * T, Gr) || !W.ok(flag.ensure(E, W.s), "alloc flags") || !W.ok(pos.ensure(E, W.s), "alloc flags"))
         return W.rc;
     sharp_flag_kernel<<<W.grid(E), 256, 0, W.s>>>(m->pn64.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, T,
                                                    angle_threshold, flag.p);
     uint64_t n = 0;
     if (!W.ok(cudaGetLastError(), "edge kernel") || !scan_u32(W, flag.p, pos.p, E, &n)) return W.rc;
-    if (!W.ok(lines.ensure(6 * std::max<uint64_t>(n, 1)), "alloc lines")) return W.rc;
+    if (!W.ok(lines.ensure(6 * std::max<uint64_t>(n, 1), W.s), "alloc lines")) return W.rc;
     sharp_emit_kernel<<<W.grid(E), 256, 0, W.s>>>(m->pn64.p, flag.p, pos.p, T, lines.p);
     if (!W.ok(cudaGetLastError(), "edge kernel")) return W.rc;
     return line_mesh(W, lines.p, n, out);
@@ -650,16 +650,16 @@ int fgc_mesh_silhouette(const fgc_mesh* m, const double eye[3], double offset, f
     if (W.rc) return W.rc;
     const uint64_t T = m->ntri;
     if (T == 0) return line_mesh(W, nullptr, 0, out);
-    DevBuf<double> nrm, seg, lines;
-    DevBuf<uint32_t> flag, pos;
-    if (!W.ok(nrm.ensure(9 * T), "alloc normals") || !W.ok(seg.ensure(6 * T), "alloc lines") ||
-        !W.ok(flag.ensure(T), "alloc flags") || !W.ok(pos.ensure(T), "alloc flags"))
+    TempBuf<double> nrm, seg, lines;
+    TempBuf<uint32_t> flag, pos;
+    if (!W.ok(nrm.ensure(9 * T, W.s), "alloc normals") || !W.ok(seg.ensure(6 * T, W.s), "alloc lines") ||
+        !W.ok(flag.ensure(T, W.s), "alloc flags") || !W.ok(pos.ensure(T, W.s), "alloc flags"))
         return W.rc;
     if (!smooth_normals_into(W, m, nrm.p)) return W.rc;  // mesh.Copy(); SmoothNormals()
     silhouette_kernel<<<W.grid(T), 256, 0, W.s>>>(m->pn64.p, nrm.p, T, eye[0], eye[1], eye[2], offset, flag.p, seg.p);
     uint64_t n = 0;
     if (!W.ok(cudaGetLastError(), "silhouette kernel") || !scan_u32(W, flag.p, pos.p, T, &n)) return W.rc;
-    if (!W.ok(lines.ensure(6 * std::max<uint64_t>(n, 1)), "alloc lines")) return W.rc;
+    if (!W.ok(lines.ensure(6 * std::max<uint64_t>(n, 1), W.s), "alloc lines")) return W.rc;
     compact_lines_kernel<<<W.grid(T), 256, 0, W.s>>>(flag.p, pos.p, seg.p, T, lines.p);
     if (!W.ok(cudaGetLastError(), "silhouette kernel")) return W.rc;
     return line_mesh(W, lines.p, n, out);
@@ -671,20 +671,17 @@ int fgc_mesh_download(const fgc_mesh* m, double* tri_pos, double* tri_nrm, doubl
     if (V == 0) return FGC_OK;
     Work W(m->device);
     if (W.rc) return W.rc;
-    DevBuf<double> pos, nrm;
-    std::vector<double> hp(3 * V), hn(3 * V);
-    if (!W.ok(pos.ensure(3 * V), "alloc") || !W.ok(nrm.ensure(3 * V), "alloc")) return W.rc;
+    TempBuf<double> pos, nrm;
+    if (!W.ok(pos.ensure(3 * V, W.s), "alloc") || !W.ok(nrm.ensure(3 * V, W.s), "alloc")) return W.rc;
     download_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, V, pos.p, nrm.p);
-    if (!W.ok(cudaGetLastError(), "download kernel") ||
-        !W.ok(cudaMemcpyAsync(hp.data(), pos.p, 3 * V * 8, cudaMemcpyDeviceToHost, W.s), "read positions") ||
-        !W.ok(cudaMemcpyAsync(hn.data(), nrm.p, 3 * V * 8, cudaMemcpyDeviceToHost, W.s), "read normals") ||
+    const uint64_t nt = 9 * m->ntri, nl = 6 * m->nline;
+    auto read = [&](double* dst, const double* src, uint64_t n) {
+        return !dst || !n || W.ok(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, W.s), "read mesh");
+    };
+    if (!W.ok(cudaGetLastError(), "download kernel") || !read(tri_pos, pos.p, nt) || !read(tri_nrm, nrm.p, nt) ||
+        !read(line_pos, pos.p + nt, nl) || !read(line_nrm, nrm.p + nt, nl) ||
         !W.ok(cudaStreamSynchronize(W.s), "download"))
         return W.rc;
-    const uint64_t nt = 9 * m->ntri, nl = 6 * m->nline;
-    if (tri_pos) std::memcpy(tri_pos, hp.data(), nt * 8);
-    if (tri_nrm) std::memcpy(tri_nrm, hn.data(), nt * 8);
-    if (line_pos) std::memcpy(line_pos, hp.data() + nt, nl * 8);
-    if (line_nrm) std::memcpy(line_nrm, hn.data() + nt, nl * 8);
     return FGC_OK;
 }
 

@@ -71,9 +71,8 @@ class DeviceMesh:
         else:
             with open(os.fspath(source), "rb") as f:
                 data = f.read()
-        buf = ctypes.create_string_buffer(data, len(data))
         h = ctypes.c_void_p()
-        _abi.check(_lib().fgc_mesh_load_stl(buf, len(data), ctypes.byref(h)))
+        _abi.check(_lib().fgc_mesh_load_stl(data, len(data), ctypes.byref(h)))  # read in place
         return cls(h.value)
 
     # -- counts --------------------------------------------------------------------
@@ -119,8 +118,8 @@ class DeviceMesh:
         """A host Mesh with this mesh's positions and normals."""
         from .mesh import Mesh
         t, l = self._counts()
-        tp, tn = np.zeros((t, 3, 3)), np.zeros((t, 3, 3))
-        lp, ln = np.zeros((l, 2, 3)), np.zeros((l, 2, 3))
+        tp, tn = np.empty((t, 3, 3)), np.empty((t, 3, 3))
+        lp, ln = np.empty((l, 2, 3)), np.empty((l, 2, 3))
         _abi.check(_lib().fgc_mesh_download(self.handle, _abi.dptr(tp), _abi.dptr(tn), _abi.dptr(lp),
                                             _abi.dptr(ln)))
         return Mesh(tp if t else None, tn if t else None, line_pos=lp if l else None, line_nrm=ln if l else None)
