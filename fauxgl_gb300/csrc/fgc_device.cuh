@@ -267,6 +267,18 @@ __device__ __forceinline__ bool dle_i(double x, double y) {
     if (bnan(bx) || bnan(by)) return false;
     return okey0(bx) <= okey0(by);
 }
+// The same for operands that are mostly non-negative (depths): their bits
+// compare as the values do, NaN lying above infinity.
+__device__ __forceinline__ bool dgt_pos(double x, double y) {
+    const unsigned long long bx = dbits(x), by = dbits(y);
+    if ((long long)(bx | by) >= 0) return bx > by && bx <= kInfBits;
+    return dgt_i(x, y);
+}
+__device__ __forceinline__ bool dle_pos(double x, double y) {
+    const unsigned long long bx = dbits(x), by = dbits(y);
+    if ((long long)(bx | by) >= 0) return bx <= by && by <= kInfBits;
+    return dle_i(x, y);
+}
 // z + bias, skipping the add for a bias of +0: z + (+0) is z, or +0 for
 // z = -0, and every use compares it, where -0 and +0 are equal.
 __device__ __forceinline__ double add_bias(double z, double bias, bool bias_zero) {
