@@ -77,6 +77,7 @@ struct PassPlan {
     int F = 0;
     int su = kSpanUnitsMin;
     int heads = kRasterHeadsMax;
+    int rounds = kChunkRounds;
     int bsize = 4;               // bytes of a fragment's barycentric (8: some draw is shaded in FP64 throughout)
     bool cert = false;           // certified shading (some draw of the plain form takes it)
     size_t smem = 0;
@@ -112,36 +113,43 @@ std::vector<std::vector<uint32_t>> split_passes(const std::vector<PassItem>& ite
     return out;
 }
 
-int fit_fragments(const DevLimits& D, const PassTuning& T, int precision, int32_t Lmax, int bsize, int& F, int& su,
-                  int& heads, size_t& smem) {
+int fit_fragments(const DevLimits& D, const PassTuning& T, int precision, int32_t Lmax, int bsize, bool large, int& F, int& su,
+                  int& heads, int& rounds, size_t& smem) {
     const int stat = D.raster_static[precision == FGC_PRECISION_MIXED ? 1 : 0];
     const long two_cta = (long)D.smem_per_sm / 2 - D.smem_reserved_per_block - stat;
     const long one_cta = (long)D.smem_per_block_optin - stat;
-    F = std::max(256, std::min(T.frag_cap, 4096));
-    heads = kRasterHeadsMax;
+    // primitives of several pixels fill a larger buffer in one round of units
+    // (kRowTablePixelsPerElement); small ones do not, and its memory is then
+    // better left to the L1 cache (raster stage at twice the cap: 48 mixed
+    // thumbnails 2.33 -> 2.13 ms, a close-up 231 -> 218 us; a dense 1080p frame at
+    // 1.5 times 295 -> 315 us)
+    F = std::max(256, std::min(large ? 2 * T.frag_cap : T.frag_cap, 4096));
+    heads = Lmax > kRasterHeadsMax ? kRasterHeadsMin : kRasterHeadsMax;
+    rounds = kChunkRounds;
     // the larger span arrays first: they also hold the warp queues of the
     // narrow walk, which needs one 32-entry queue per warp (kSpanUnitsMax =
     // the CTA's threads) and is worth more than a larger fragment buffer
     su = kSpanUnitsMax;
-    smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+    smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
     // two CTAs per SM (the register budget allows two) when a smaller
     // fragment buffer makes them fit
     while ((long)smem > two_cta && F > 512) {
         F -= 128;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
     }
     while ((long)smem > one_cta && F > 256) {
         F /= 2;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
     }
     if ((long)smem > one_cta) {
         heads = kRasterHeadsMin;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+        rounds = 1;
+        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
     }
     if ((long)smem > one_cta) {
         // the smaller span arrays (narrow rows then walk thread by thread)
         su = kSpanUnitsMin;
-        smem = raster_smem_bytes(Lmax, F, kRasterThreads, su, heads, bsize);
+        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
     }
     if (Lmax > kBandPixelsMax || (long)smem > one_cta) return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
     return FGC_OK;
@@ -268,7 +276,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     P.band[n] = P.nbands;
     if (P.nmat >= 0xFFFFFFFFull) return fail(FGC_ERR_UNSUPPORTED, "pass too large for its bin matrix");
     P.scan_tiles = (uint32_t)ceil_div(P.nmat, 2048);
-    int rc = fit_fragments(D, T, P.precision, P.Lmax, P.bsize, P.F, P.su, P.heads, P.smem);
+    int rc = fit_fragments(D, T, P.precision, P.Lmax, P.bsize, P.row_table, P.F, P.su, P.heads, P.rounds, P.smem);
     if (rc) return rc;
     const int warps = (int)std::min<int64_t>(8, (96 * 1024) / ((int64_t)P.max_nbands * 4));
     if (warps < 1) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands for binning");
@@ -651,6 +659,7 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.F = P.F;
         rp.bsize = P.bsize;
         rp.heads = P.heads;
+        rp.rounds = P.rounds;
         rp.Lmax = P.Lmax;
         rp.su = P.su;
         rp.pend = P.cert ? S.pend.p : nullptr;

@@ -45,16 +45,14 @@ struct RasterSmem {
     double* bd;      // [3][F] for FP64 shading of every fragment (exact)
     int fcap;        // F
     uint32_t* fkey;  // [F] (pixel << 16) | unit
-    uint32_t* fcol;  // [F] NRGBA
     double* uw0;     // [su] unit -> edge values at its first covered in-band pixel
     double* uw1;
     double* uw2;
-    uint32_t* uslot; // [kRT] unit -> chunk slot
-    int32_t* urow;   // [kRT] unit -> row y
+    uint32_t* uprim; // [P.rounds * kRT] unit -> primitive
+    int32_t* urow;   // [P.rounds * kRT] unit -> row y
     int32_t* ux;     // [su] unit -> first covered in-band x
     uint32_t* ucnt;  // [su] unit -> covered in-band pixels
     uint32_t* ufrag; // [su] unit -> first fragment offset in the chunk
-    uint32_t* cprim; // [kChunkPrims] chunk slot -> primitive
     unsigned short* head;  // [kHeads] per pixel bucket: last fragment of its list (0xFFFF: none)
     unsigned short* nxt;   // [F] per fragment: the previous fragment in its bucket
     uint8_t* fflag;  // [F] discard / blend / pending flags
@@ -63,6 +61,10 @@ struct RasterSmem {
     uint32_t mark;   // colour word of a pixel whose colour is pending, entry 0
     bool exact;      // the draw's fragments are shaded in FP64, every one
     uint32_t hmask;  // pixel buckets - 1
+    // a shaded fragment's NRGBA, in the place of its own first barycentric
+    __device__ __forceinline__ uint32_t& col(uint32_t f) const {
+        return reinterpret_cast<uint32_t*>(bf)[exact ? 2 * f : f];
+    }
     __device__ __forceinline__ uint32_t bucket(uint32_t pix) const { return pix & hmask; }
 };
 
@@ -566,7 +568,7 @@ __device__ __noinline__ uint32_t quad_span(const RasterParams& P, const ItemView
     int32_t x0 = 0, x1 = -1, rel = 0;
     unsigned long long skip = 0;  // this edge's share of d: a non-negative double
     if (has) {
-        const uint32_t pp = S.cprim[S.uslot[u]];
+        const uint32_t pp = S.uprim[u];
         const int32_t y = S.urow[u];
         const RPrim& R = P.prims[pp];
         const PBox bx = P.pbox[pp];
@@ -923,7 +925,7 @@ __device__ __forceinline__ void quad_run(const RasterParams& P, const ItemView& 
             const uint32_t o = off - S.ufrag[u];
             left = S.ucnt[u] - o;
             pix = (S.urow[u] - B.r0) * I.W + S.ux[u] + (int32_t)o;
-            const RPrim& R = P.prims[S.cprim[S.uslot[u]]];
+            const RPrim& R = P.prims[S.uprim[u]];
             a = (&R.a0)[e];
             ra = R.ra;
             z0 = R.z0;
@@ -1002,28 +1004,28 @@ __device__ __forceinline__ void apply_fragment(const RasterParams& P, const Item
                     cc.v = *cp;
                     cc.loaded = true;
                 }
-                cc.v = blend_nrgba(cc.v, S.fcol[f]);
+                cc.v = blend_nrgba(cc.v, S.col(f));
                 cc.dirty = true;
             } else {
                 // SetNRGBA(x, y, c) ignores points outside the image rectangle:
                 // x = i - y*W with i = r0*W + pix
                 const int32_t x = pix - (S.urow[unit] - B.r0) * I.W;
                 if (x >= 0 && x < I.W) {
-                    cc.v = S.fcol[f];
+                    cc.v = S.col(f);
                     cc.loaded = true;
                     cc.dirty = true;
                     if (fl == kFragPending) {
                         // the pixel holds the entry's mark until the list is
                         // emptied, unless a later fragment takes the pixel
                         const uint32_t e = atomicAdd(S.npend, 1u);  // the chunk was checked to fit
-                        S.pend[e] = PendFrag{S.cprim[S.uslot[unit]], S.urow[unit], (uint32_t)pix};
+                        S.pend[e] = PendFrag{S.uprim[unit], S.urow[unit], (uint32_t)pix};
                         cc.v = S.mark + e;
                     }
                 }
             }
         }
         if (I.winner) {
-            const uint32_t p = S.cprim[S.uslot[unit]];
+            const uint32_t p = S.uprim[unit];
             I.winner[B.i0 + pix] = P.prims[p].elem;
         }
         if (I.shaded) {
@@ -1102,7 +1104,7 @@ template <int PREC>
 __device__ __forceinline__ void shade_fragment(const RasterParams& P, const ItemView& I, RasterSmem& S, uint32_t f,
                                                uint32_t* s_fresh) {
     const uint32_t unit = S.fkey[f] & 0xffff;
-    const uint32_t prim = S.cprim[S.uslot[unit]];
+    const uint32_t prim = S.uprim[unit];
     const RPrim& R = P.prims[prim];
     uint8_t fl = 0;
     if (PREC == FGC_PRECISION_PLAIN && S.pend) {
@@ -1111,7 +1113,7 @@ __device__ __forceinline__ void shade_fragment(const RasterParams& P, const Item
             fl = kFragPending;
             atomicAdd(s_fresh, 1u);
         }
-        S.fcol[f] = out;
+        S.col(f) = out;
         S.fflag[f] = fl;
         return;
     }
@@ -1135,7 +1137,7 @@ __device__ __forceinline__ void shade_fragment(const RasterParams& P, const Item
         packed = u8_of_unit_f32(col.x) | (u8_of_unit_f32(col.y) << 8) | (u8_of_unit_f32(col.z) << 16) |
                  (u8_of_unit_f32(col.w) << 24);
     }
-    S.fcol[f] = packed;
+    S.col(f) = packed;
     S.fflag[f] = fl;
     if (P.dbg) {
         double* dst = P.dbg + ((uint64_t)blockIdx.x * P.F + f) * 4;
@@ -1357,19 +1359,18 @@ __global__ void __launch_bounds__(kRT, 2) raster_kernel(RasterParams P) {
         S.depth = (double*)q; q += (size_t)P.Lmax * 8;
         S.fz = (double*)q; q += (size_t)F * 8;
         S.bf = (float*)q;
-        S.bd = (double*)q; q += (size_t)F * 3 * P.bsize;
+        S.bd = (double*)q;
+        q += (size_t)F * 3 * P.bsize;
         S.fcap = F;
         S.uw0 = (double*)q; q += (size_t)P.su * 8;
         S.uw1 = (double*)q; q += (size_t)P.su * 8;
         S.uw2 = (double*)q; q += (size_t)P.su * 8;
         S.fkey = (uint32_t*)q; q += (size_t)F * 4;
-        S.fcol = (uint32_t*)q; q += (size_t)F * 4;
-        S.uslot = (uint32_t*)q; q += kRT * 4;
-        S.urow = (int32_t*)q; q += kRT * 4;
+        S.uprim = (uint32_t*)q; q += (size_t)P.rounds * kRT * 4;
+        S.urow = (int32_t*)q; q += (size_t)P.rounds * kRT * 4;
         S.ux = (int32_t*)q; q += (size_t)P.su * 4;
         S.ucnt = (uint32_t*)q; q += (size_t)P.su * 4;
         S.ufrag = (uint32_t*)q; q += (size_t)P.su * 4;
-        S.cprim = (uint32_t*)q; q += kChunkPrims * 4;
         S.head = (unsigned short*)q; q += (size_t)P.heads * 2;
         S.hmask = (uint32_t)P.heads - 1;
         S.nxt = (unsigned short*)q; q += (size_t)F * 2;
@@ -1440,142 +1441,156 @@ __global__ void __launch_bounds__(kRT, 2) raster_kernel(RasterParams P) {
         EntryLoad pf;
         uint32_t roff = 0;  // rows of the entry at k taken by earlier chunks
         int level = 0;      // 0: estimated fragments, 1: widest-chord bound, 2: box bound
-        while (k < bcount) {
-            // ---- chunk: a prefix of the remaining bin; thread t examines
-            // entries k + kChunkPer*t + j. The first primitive picks how the
-            // chunk is walked:
+        // The open chunk: rounds of direct units walked so far, whose fragments
+        // wait for the shade and resolve phases.
+        int rounds = 0;
+        uint32_t ubase = 0;     // their units
+        uint64_t kopen = 0;     // where it began (entry, rows of it taken before): a chunk
+        uint32_t ropen = 0;     //   that outgrows F is redone from there
+        uint64_t topen = 0;     // this thread's covered pixels of its rounds
+        for (;;) {
+            // ---- round: a prefix of the remaining bin; thread t examines
+            // entry k + t. The first primitive picks how it is walked:
             //   direct  narrow primitives, each row walked and recorded by one
-            //           thread as rasterize does, up to F units. The prefix
-            //           keeps an estimate of its fragments within F: at level
-            //           0 the bound (rows x widest chord) scaled by the share
-            //           of bounded pixels that became fragments in earlier
-            //           chunks (early depth rejection makes it small); a walk
-            //           that outgrows F is redone at level 1 with the bound
-            //           itself, then at level 2 with the box width
+            //           thread as rasterize does, up to a unit per thread. The
+            //           prefix keeps an estimate of its fragments within what
+            //           is left of F: at level 0 the bound (rows x widest
+            //           chord) scaled by the share of bounded pixels that
+            //           became fragments in earlier chunks (early depth
+            //           rejection makes it small); a walk that outgrows F is
+            //           redone at level 1 with the bound itself, then at level
+            //           2 with the box width. A chunk takes up to
+            //           P.rounds direct rounds while their fragments fit,
+            //           so that the phases after the walk -- mostly latency and
+            //           barriers -- are paid once for them.
             //   spans   anything else, at most P.su units: spans, then
-            //           windows of fragment offsets
-            // An entry with more rows in the band than its chunk holds (rows
+            //           runs of fragment offsets; a chunk of its own
+            // An entry with more rows in the band than a round holds (rows
             // that wrap around the frame's sides) goes alone, its rows over
             // several chunks.
-            const uint64_t e0 = k + (uint64_t)threadIdx.x * kChunkPer;
-            ChunkEntry ce[kChunkPer];
-#pragma unroll
-            for (int j = 0; j < kChunkPer; j++) {
-                if (e0 + j < bcount) {
-                    const EntryLoad l = (j == 0 && pf_at == e0) ? pf : load_entry(P, bstart + e0 + j);
-                    ce[j] = chunk_entry(I, B, l, level == 2, (e0 + j == k) ? roff : 0u);
-                } else {
-                    ce[j] = ChunkEntry{0, 0, 0, 0, true};
+            if (k >= bcount && rounds == 0) break;
+            bool direct = false, close = k >= bcount;  // close: shade and resolve the open chunk now
+            uint32_t split = 0, nprim = 0, nunit = 0;  // split: rows of the entry at k taken when it goes alone
+            if (!close) {
+                const uint64_t e0 = k + threadIdx.x;
+                ChunkEntry ce{0, 0, 0, 0, true};
+                if (e0 < bcount) {
+                    const EntryLoad l = pf_at == e0 ? pf : load_entry(P, bstart + e0);
+                    ce = chunk_entry(I, B, l, level == 2, e0 == k ? roff : 0u);
                 }
-            }
-            if (threadIdx.x == 0) {
-                const bool dm = ce[0].narrow && ce[0].bound <= (uint32_t)F;
-                // a direct chunk holds at most one unit per thread: a second
-                // pass over the units would double its first warps' walk
-                const uint32_t cap0 = dm ? (uint32_t)min(F, kRT) : (uint32_t)P.su;
-                s_mode = dm ? 1u : 0u;
-                s_split = ((uint32_t)ce[0].nrows > cap0) ? cap0 : 0u;
-                s_nprim = 0;
-                s_nunit = 0;
-                s_bsum = 0;
-            }
-            __syncthreads();
-            const bool direct = s_mode != 0;
-            const uint32_t split = s_split;  // rows of the entry at k this chunk takes, when it goes alone
-            const uint32_t ratio = level == 0 ? s_ratio : kRatioOne;
-            const uint64_t ucap = direct ? (uint64_t)min(F, kRT) : (uint64_t)P.su;
-            const int jmax = split ? (threadIdx.x == 0 ? 1 : 0) : kChunkPer;
-            if (split && threadIdx.x == 0) ce[0].nrows = (int32_t)split;
-            // the fragment estimates and the units in one scan (estimates in
-            // the high half, units in the low half). An entry whose estimate
-            // is above F, or whose rows are more than the chunk's units, ends
-            // the chunk wherever it stands, so each value is capped at one
-            // above its limit: every comparison below is unchanged, and both
-            // sums stay far below 2^32 (256 entries per chunk)
-            uint64_t tkey = 0, tun = 0;
-#pragma unroll
-            for (int j = 0; j < kChunkPer; j++) {
-                if (j >= jmax) break;
-                tkey += min(chunk_key(ce[j], direct, ratio, F), (uint64_t)F + 1);
-                tun += min((uint64_t)ce[j].nrows, ucap + 1);
-            }
-            uint64_t pagg;
-            const uint64_t pr = block_exclusive_scan<kRT>((tkey << 32) | tun, s_warp, &pagg);
-            uint64_t kr = pr >> 32, ur = pr & 0xffffffffull;
-            // the entries inside the prefix (never empty: the first entry's
-            // rows fit, and a direct chunk's first estimate is at most its
-            // bound <= F)
-            {
-                const uint64_t ur0 = ur;
-                uint32_t took = 0, bsum = 0;
-#pragma unroll
-                for (int j = 0; j < kChunkPer; j++) {
-                    if (j >= jmax) break;
-                    const uint64_t key = min(chunk_key(ce[j], direct, ratio, F), (uint64_t)F + 1);
-                    if (e0 + j >= bcount || ur + (uint64_t)ce[j].nrows > ucap || kr + key > (uint64_t)F) break;
-                    const uint32_t slot = threadIdx.x * kChunkPer + j;
-                    S.cprim[slot] = ce[j].p;
-                    for (int r = 0; r < ce[j].nrows; r++) {
-                        S.uslot[ur + r] = slot;
-                        S.urow[ur + r] = ce[j].ylo + r;
-                    }
-                    kr += key;
-                    ur += (uint64_t)ce[j].nrows;
-                    took++;
-                    bsum += min(ce[j].bound, (uint32_t)F);
-                }
-                if (took) {
-                    atomicAdd(&s_nprim, took);
-                    atomicAdd(&s_nunit, (uint32_t)(ur - ur0));
-                    atomicAdd(&s_bsum, bsum);
-                }
-            }
-            __syncthreads();
-            const uint32_t nprim = s_nprim, nunit = s_nunit;
-
-            if (direct) {
                 if (threadIdx.x == 0) {
-                    s_nfrag = 0;
-                    s_conflict = 0;
-                    s_fresh = 0;
-                    s_held = s_npend;
-                }
-                __syncthreads();
-                uint64_t tchunk = 0;
-                if (P.su >= kRT) {
-                    // the span arrays hold a 32-entry queue per warp: every
-                    // thread takes part, a unit each (nunit <= kRT here)
-                    const uint32_t u = threadIdx.x;
-                    const bool has = u < nunit;
-                    const uint32_t pp = has ? S.cprim[S.uslot[u]] : 0u;
-                    tchunk += walk_rows_queued<PREC>(has, pp, P.prims[pp], P.pbox[pp], has ? S.urow[u] : 0, P, I, B, S, u,
-                                               &s_nfrag, &s_conflict, vis);
-                } else {
-                    for (uint32_t u = threadIdx.x; u < nunit; u += blockDim.x) {
-                        const uint32_t pp = S.cprim[S.uslot[u]];
-                        tchunk += walk_row<PREC>(pp, P.prims[pp], P.pbox[pp], S.urow[u], P, I, B, S, u, &s_nfrag,
-                                           &s_conflict, vis);
-                    }
-                }
-                {
-                    // the next chunk's entries load during this one's shading
-                    // and resolve (a redone chunk reloads)
-                    const uint64_t nk = (split ? k : k + nprim) + threadIdx.x;
-                    if (nk < bcount) {
-                        pf = load_entry(P, bstart + nk);
-                        pf_at = nk;
+                    const bool dm = ce.narrow && ce.bound <= (uint32_t)F;
+                    // a direct round holds at most one unit per thread: a second
+                    // pass over the units would double its first warps' walk
+                    const uint32_t cap0 = dm ? (uint32_t)min(F, kRT) : (uint32_t)P.su;
+                    s_mode = dm ? 1u : 0u;
+                    s_split = ((uint32_t)ce.nrows > cap0) ? cap0 : 0u;
+                    s_nprim = 0;
+                    s_nunit = 0;
+                    if (rounds == 0) {
+                        s_bsum = 0;
+                        s_nfrag = 0;
+                        s_conflict = 0;
+                        s_fresh = 0;
+                        s_held = s_npend;
                     }
                 }
                 __syncthreads();
-                const bool redo = (s_conflict & 2u) != 0;
+                direct = s_mode != 0;
+                split = s_split;
+                close = rounds != 0 && (!direct || split != 0);
+                if (!close) {
+                    const uint32_t ratio = level == 0 ? s_ratio : kRatioOne;
+                    const uint64_t room = (uint64_t)F - (rounds ? s_nfrag : 0u);  // s_nfrag <= F: an outgrown chunk was redone
+                    const uint64_t ucap = direct ? (uint64_t)min(F, kRT) : (uint64_t)P.su;
+                    const bool mine = e0 < bcount && (!split || threadIdx.x == 0);
+                    if (split && threadIdx.x == 0) ce.nrows = (int32_t)split;
+                    // the fragment estimates and the units in one scan
+                    // (estimates in the high half, units in the low half). An
+                    // entry whose estimate is above F, or whose rows are more
+                    // than the round's units, ends the round wherever it
+                    // stands, so each value is capped at one above its limit:
+                    // every comparison below is unchanged, and both sums stay
+                    // far below 2^32 (256 entries per round)
+                    const uint64_t key = mine ? min(chunk_key(ce, direct, ratio, F), (uint64_t)F + 1) : 0;
+                    const uint64_t tun = mine ? min((uint64_t)ce.nrows, ucap + 1) : 0;
+                    uint64_t pagg;
+                    const uint64_t pr = block_exclusive_scan<kRT>((key << 32) | tun, s_warp, &pagg);
+                    const uint64_t kr = pr >> 32, ur = pr & 0xffffffffull;
+                    // the entries inside the prefix (not empty in a chunk's
+                    // first round: the first entry's rows fit, and a direct
+                    // round's first estimate is at most its bound <= F)
+                    if (mine && ur + (uint64_t)ce.nrows <= ucap && kr + key <= room) {
+                        for (int r = 0; r < ce.nrows; r++) {
+                            S.uprim[ubase + ur + r] = ce.p;
+                            S.urow[ubase + ur + r] = ce.ylo + r;
+                        }
+                        atomicAdd(&s_nprim, 1u);
+                        atomicAdd(&s_nunit, (uint32_t)ce.nrows);
+                        atomicAdd(&s_bsum, min(ce.bound, (uint32_t)F));
+                    }
+                    __syncthreads();
+                    nprim = s_nprim;
+                    nunit = s_nunit;
+                    close = rounds != 0 && nprim == 0;
+                }
+            }
+
+            if (close || direct) {
+                bool redo = false;
+                if (!close) {
+                    if (rounds == 0) {
+                        kopen = k;
+                        ropen = roff;
+                    }
+                    if (P.su >= kRT) {
+                        // the span arrays hold a 32-entry queue per warp: every
+                        // thread takes part, a unit each (nunit <= kRT here)
+                        const uint32_t u = ubase + threadIdx.x;
+                        const bool has = threadIdx.x < nunit;
+                        const uint32_t pp = has ? S.uprim[u] : 0u;
+                        topen += walk_rows_queued<PREC>(has, pp, P.prims[pp], P.pbox[pp], has ? S.urow[u] : 0, P, I, B, S,
+                                                        u, &s_nfrag, &s_conflict, vis);
+                    } else {
+                        for (uint32_t u = ubase + threadIdx.x; u < ubase + nunit; u += blockDim.x) {
+                            const uint32_t pp = S.uprim[u];
+                            topen += walk_row<PREC>(pp, P.prims[pp], P.pbox[pp], S.urow[u], P, I, B, S, u, &s_nfrag,
+                                                    &s_conflict, vis);
+                        }
+                    }
+                    {
+                        // the next round's entries load meanwhile (a redone
+                        // chunk reloads)
+                        const uint64_t nk = (split ? k : k + nprim) + threadIdx.x;
+                        if (nk < bcount) {
+                            pf = load_entry(P, bstart + nk);
+                            pf_at = nk;
+                        }
+                    }
+                    __syncthreads();
+                    redo = (s_conflict & 2u) != 0;
+                    rounds++;
+                    ubase += nunit;
+                    if (split) {
+                        roff += split;
+                    } else {
+                        k += nprim;
+                        roff = 0;
+                    }
+                    // another round while the buffer fills by less than a
+                    // quarter in each (a round that has to stop short of a
+                    // unit per thread walks no faster for it)
+                    if (!redo && split == 0 && level == 0 && rounds < P.rounds && k < bcount &&
+                        s_nfrag * 4 <= (uint32_t)F * (uint32_t)rounds)
+                        continue;
+                }
+                const uint32_t nfrag = min(s_nfrag, (uint32_t)F);
                 if (redo) {  // nothing was applied: empty the lists, redo with a safer bound
-                    const uint32_t nrec = min(s_nfrag, (uint32_t)F);
-                    for (uint32_t f = threadIdx.x; f < nrec; f += blockDim.x)
+                    for (uint32_t f = threadIdx.x; f < nfrag; f += blockDim.x)
                         S.head[S.bucket(S.fkey[f] >> 16)] = 0xFFFFu;
                     if (threadIdx.x == 0) s_ratio = kRatioOne;
                 } else {
-                    tot += tchunk;
-                    const uint32_t nfrag = s_nfrag;
+                    tot += topen;
                     if (threadIdx.x == 0) {
                         shd += nfrag;
                         s_ratio = next_ratio(s_ratio, nfrag, s_bsum);
@@ -1589,18 +1604,17 @@ __global__ void __launch_bounds__(kRT, 2) raster_kernel(RasterParams P) {
                     resolve_chunk(P, I, B, S, nfrag, (s_conflict & 1u) != 0, upd, &s_rank);
                 }
                 __syncthreads();
+                rounds = 0;
+                ubase = 0;
+                topen = 0;
                 if (redo && level < 2) {
                     level++;
+                    k = kopen;
+                    roff = ropen;
                     continue;
                 }
                 if (redo && threadIdx.x == 0) atomicOr(P.status, ST_RASTER_INTERNAL);
                 level = 0;
-                if (split) {
-                    roff += split;
-                } else {
-                    k += nprim;
-                    roff = 0;
-                }
                 continue;
             }
             level = 0;
