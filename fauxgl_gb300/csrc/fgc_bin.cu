@@ -80,7 +80,13 @@ __global__ void __launch_bounds__(256) bin_count_kernel(BinParams P) {
 // exact serial sum, fgc_fpjump.cuh) and adds row by row from there, so a
 // tall primitive no longer holds its warp while the others' lanes idle.
 // Gaps above 64 rows between bands are crossed with exact jumps as well.
-constexpr uint32_t kRowSeg = 8;
+// A pass of few primitives is spread over the grid, down to kRowTileMin of
+// them per block: five blocks of 256 had the 1,232 primitives of a close-up
+// frame to themselves, 114 us; 154 blocks of 8 take 41 us. (Segments of 8
+// bands instead of 16 jump twice as often: 25.5 M pairs of a wireframe overlay
+// 600 -> 500 us; of 4 they took 910 us.)
+constexpr uint32_t kRowSeg = 16;
+constexpr uint32_t kRowTile = 256;    // primitives per block at most (its threads)
 
 __device__ __forceinline__ double row_advance(double w, double b, int64_t gap) {
     if (gap > 64) return repeat_add(w, b, (uint64_t)gap);
@@ -98,16 +104,17 @@ __global__ void __launch_bounds__(256) row_starts_kernel(RowStartParams P) {
     __syncthreads();
     if (s_stop) return;
     const uint64_t n = *P.prim_total;
-    for (uint64_t t0 = (uint64_t)blockIdx.x * 256; t0 < n; t0 += (uint64_t)gridDim.x * 256) {
+    const uint32_t tile = (uint32_t)min((uint64_t)kRowTile, max((uint64_t)kRowTileMin, (n + gridDim.x - 1) / gridDim.x));
+    for (uint64_t t0 = (uint64_t)blockIdx.x * tile; t0 < n; t0 += (uint64_t)gridDim.x * tile) {
         const uint64_t p0 = t0 + threadIdx.x;
-        const uint32_t cnt0 = p0 < n ? P.pnb[p0] : 0u;
+        const uint32_t cnt0 = p0 < n && threadIdx.x < tile ? P.pnb[p0] : 0u;
         uint64_t total;
         const uint64_t first = block_exclusive_scan<256>((cnt0 + kRowSeg - 1) / kRowSeg, s_warp, &total);
         s_seg[threadIdx.x] = (uint32_t)first;
         __syncthreads();
         for (uint32_t sg = threadIdx.x; sg < (uint32_t)total; sg += blockDim.x) {
             // the primitive holding segment sg: the last one starting at or before it
-            uint32_t lo = 0, hi = 255;
+            uint32_t lo = 0, hi = tile - 1;
             while (lo < hi) {
                 const uint32_t mid = (lo + hi + 1) >> 1;
                 if (s_seg[mid] <= sg) lo = mid;

@@ -222,6 +222,9 @@ struct ScanParams {
     const unsigned long long* n_dev;  // when set, only the first min(n, *n_dev) values are scanned
 };
 
+// Primitives per row-start block at least.
+constexpr uint32_t kRowTileMin = 8;
+
 // Primitives with boxes at most this many rows tall catch up their rows from
 // the top themselves; taller ones have row starts per band.
 constexpr int32_t kRowTableMinRows = 5;

@@ -88,6 +88,13 @@ struct PassPlan {
 };
 
 constexpr double kRowTablePixelsPerElement = 8.0;
+// Primitives of a binning block at least, and blocks of a draw as far as that
+// allows. Few tall primitives make many (primitive, band) pairs: a close-up of
+// 1,232 of them (19,302 pairs) was counted and placed by 2 blocks in 111 us, in a
+// batch of 20 supersampled thumbnails most draws had one block (binning with
+// row starts 580 us, 260 with up to 32 blocks).
+constexpr int64_t kBinPrimsMin = 16;
+constexpr uint64_t kBinBlocksMin = 32;
 
 uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
@@ -172,7 +179,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     // 128x128 223 -> 41 us, 1280x720 197 -> 166 us, though primitives meet more
     // bands. Below that smaller bands no longer pay (1080p at one row a band:
     // 293 -> 305 us). Binning 81,920 triangles in 20 blocks of 4,096 took 61 us,
-    // in 304 39 us; below 256 primitives a block there is nothing left to gain.
+    // in 304 39 us.
     uint64_t pass_px = 0, pass_prims = 0;
     for (uint32_t i : idx) {
         const PassItem& it = sub.items[i];
@@ -181,7 +188,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     }
     const int64_t band_pixels = std::min<int64_t>(T.band_pixels, (int64_t)(pass_px / (2 * (uint64_t)D.sms)));
     const int64_t bin_prims =
-        std::min<int64_t>(T.prims_per_bin_block, std::max<int64_t>(256, (int64_t)(pass_prims / (2 * (uint64_t)D.sms))));
+        std::min<int64_t>(T.prims_per_bin_block, std::max<int64_t>(kBinPrimsMin, (int64_t)(pass_prims / (2 * (uint64_t)D.sms))));
     for (uint32_t j = 0; j < n; j++) {
         const PassItem& it = sub.items[idx[j]];
         const fgc_context* c = it.ctx;
@@ -209,7 +216,8 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
         if (v.nbands > (uint32_t)kMaxBands) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands");
         const int per = it.sv.wireframe ? 6 : 1;
         const uint64_t prims = it.tc * per + it.lc * 2;
-        v.nblk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, ceil_div(prims, (uint64_t)bin_prims)),
+        const uint64_t per_blk = std::min<uint64_t>(bin_prims, std::max<uint64_t>(kBinPrimsMin, prims / kBinBlocksMin));
+        v.nblk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, ceil_div(prims, per_blk)),
                                               (uint64_t)2 * D.sms);
         const bool draws = it.tc > 0 || it.lc > 0;
         const uint32_t vt = draws ? (uint32_t)ceil_div(it.mesh->nuniq, kVertexTile) : 0;
@@ -635,7 +643,7 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
             rq.cap = S.bin_cap;
             rq.rstart = S.rstart.p;
             rq.status = status;
-            row_starts_kernel<<<grid_for(prim_cap0, 256, D.sms * 8), 256, 0, stream>>>(rq);
+            row_starts_kernel<<<grid_for(prim_cap0, kRowTileMin, D.sms * 8), 256, 0, stream>>>(rq);
             FGC_CUDA(cudaGetLastError());
             rec.launches += 2;
         }
