@@ -33,13 +33,13 @@ int grid_for(uint64_t n, int block, int cap) {
 }
 
 // ---------------------------------------------------------------------------
-// Mesh memory pools and call streams, one set per device
+// Memory pools and call streams, one set per device
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kMaxDevices = 64;
 constexpr size_t kKeptStreams = 8;
 struct DevicePool {
-    cudaMemPool_t pool = nullptr;
+    cudaMemPool_t pool[kPoolKinds] = {};
     cudaStream_t free_stream = nullptr;
     std::vector<cudaStream_t> idle;
 };
@@ -53,48 +53,46 @@ cudaError_t device_pool(DevicePool** out) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     DevicePool& P = g_pools[dev];
-    if (!P.pool) {
+    if (!P.free_stream) {
         cudaMemPoolProps props;
         memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        e = cudaMemPoolCreate(&pool, &props);
-        if (e != cudaSuccess) return e;
-        uint64_t keep = kPoolKeep;
-        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        for (int k = 0; k < kPoolKinds && e == cudaSuccess; k++) {
+            if (P.pool[k]) continue;  // of an attempt that failed further on
+            e = cudaMemPoolCreate(&P.pool[k], &props);
+            uint64_t keep = kPoolKeep;
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(P.pool[k], cudaMemPoolAttrReleaseThreshold, &keep);
+        }
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P.free_stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) {
-            cudaMemPoolDestroy(pool);
+            P.free_stream = nullptr;
             return e;
         }
-        P.pool = pool;
     }
     *out = &P;
     return cudaSuccess;
 }
 }  // namespace
 
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+cudaError_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s) {
     DevicePool* P = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
         const cudaError_t e = device_pool(&P);
         if (e != cudaSuccess) return e;
     }
-    return cudaMallocFromPoolAsync(p, bytes, P->pool, s);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, P->pool[kind], s);
+    if (e == cudaErrorMemoryAllocation) {  // with the other pools' spare memory
+        cudaGetLastError();
+        for (cudaMemPool_t pool : P->pool) cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, P->pool[kind], s);
+    }
+    return e;
 }
 
 void pool_free(void* p, cudaStream_t s) { cudaFreeAsync(p, s); }
-
-bool pool_trim() {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    bool any = false;
-    for (DevicePool& P : g_pools)
-        if (P.pool) any = cudaMemPoolTrimTo(P.pool, 0) == cudaSuccess || any;
-    return any;
-}
 
 cudaError_t take_stream(int device, cudaStream_t* s) {
     {

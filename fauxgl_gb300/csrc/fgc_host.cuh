@@ -33,21 +33,23 @@ int fail(int code, const std::string& msg);
         if (e_ != cudaSuccess) return ::fgc::fail(FGC_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Mesh memory: the arrays of meshes and the temporaries of the calls that
-// make and edit them come from one stream-ordered pool per device. A call
-// allocates up to two dozen arrays; cudaMalloc and cudaFree (which waits for
-// the device) took most of its time: LoadSTL of 327,680 triangles 2.8 ms,
-// SmoothNormals 1.3 ms, a mesh of 81,920 uploaded for one draw 1.6 ms; from the
-// pool they take 0.29, 0.26 and 0.28 ms. The pool keeps at most kPoolKeep bytes of freed
-// memory (the driver returns the rest when a stream synchronises), and gives
-// all of it back when an allocation outside the pool fails. It is the
-// driver's, so threads and streams may use it together: memory freed on one
+// Device memory comes from stream-ordered pools, three per device: the
+// temporaries of the calls that make and edit meshes, the arrays of meshes,
+// and everything else (framebuffers, a context's or batch's scratch).
+// cudaMalloc and cudaFree (which waits for the device) took most of the time
+// of mesh calls, which allocate up to two dozen arrays: LoadSTL of 327,680
+// triangles 2.8 ms, SmoothNormals 1.3 ms, a mesh of 81,920 uploaded for one
+// draw 1.6 ms; from the pools they take 0.29, 0.26 and 0.28 ms. The first draw
+// into a new 1080p context, which allocates its scratch, takes 1.27 ms instead
+// of 2.36. Each pool keeps at most kPoolKeep bytes of freed memory (the driver
+// returns the rest when a stream synchronises), so that many resident meshes
+// or large frames do not take the temporaries' share. The pools are the
+// driver's, so threads and streams may use them together: memory freed on one
 // stream is handed to another only once that free has taken effect.
 constexpr uint64_t kPoolKeep = 1ull << 30;
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
+enum PoolKind { kPoolTemp, kPoolMesh, kPoolFrame, kPoolKinds };
+cudaError_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s);
 void pool_free(void* p, cudaStream_t s);
-// Give the pools' spare memory back; false when there is no pool yet.
-bool pool_trim();
 // A stream of the device for one call (kept for later calls, at most eight)
 // and its return. free_stream: the stream on which memory outliving its call
 // is freed, after the device has been waited for.
@@ -76,7 +78,7 @@ struct PoolBuf {
         release();
         s = stream;
         const size_t want = std::max<size_t>(n, 1);
-        const cudaError_t e = pool_alloc((void**)&p, want * sizeof(T), stream);
+        const cudaError_t e = pool_alloc(Kept ? kPoolMesh : kPoolTemp, (void**)&p, want * sizeof(T), stream);
         if (e != cudaSuccess) {
             p = nullptr;
             return e;
@@ -90,6 +92,8 @@ using TempBuf = PoolBuf<T, false>;
 template <typename T>
 using MeshBuf = PoolBuf<T, true>;
 
+// A buffer that any stream may use: the device is waited for before it is
+// freed, and its allocation has taken effect before it is used.
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
@@ -99,7 +103,10 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p) {
+            cudaDeviceSynchronize();
+            pool_free(p, free_stream());
+        }
         p = nullptr;
         cap = 0;
     }
@@ -108,11 +115,9 @@ struct DevBuf {
         if (n <= cap && p) return cudaSuccess;
         release();
         size_t want = std::max<size_t>(n + n / 4, 64);
-        cudaError_t e = cudaMalloc((void**)&p, want * sizeof(T));
-        if (e == cudaErrorMemoryAllocation && pool_trim()) {  // the mesh pool's spare memory first
-            cudaGetLastError();
-            e = cudaMalloc((void**)&p, want * sizeof(T));
-        }
+        const cudaStream_t s = free_stream();
+        cudaError_t e = pool_alloc(kPoolFrame, (void**)&p, want * sizeof(T), s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             p = nullptr;
             return e;
