@@ -160,18 +160,60 @@ __global__ void group_sort_kernel(const uint32_t* start, const uint32_t* count, 
 // in corner order, of the group's normals whose dot product with the
 // corner's own is at least the threshold. A NaN position finds no group: the
 // sum is the zero vector and normalises to NaN.
-__global__ void smooth_threshold_kernel(const APosNrm64* pn, const uint32_t* gid, const uint32_t* start,
-                                        const uint32_t* count, const uint32_t* member, uint64_t V, double threshold,
-                                        double* out) {
+//
+// FP64-bound at ~70 operations a corner (147 us for 983,040). Whether a dot
+// product reaches the threshold is decided in FP32 where it is further from
+// it than FP32 can be off (side_of); and where every pair of a group's normals
+// reaches it -- a smooth place -- all its corners have the same sum, formed
+// once (smooth_shared_kernel). SMOOTH_AFTER us for both.
+
+// +1: the FP64 dot product of the normals behind a and b is at least thr, -1:
+// below it, 0: too near to tell. The FP32 dot product of rounded components is
+// within 6 * 2^-24 of the sum of its products' sizes; thr is rounded once.
+__device__ __forceinline__ int side_of(const APosNrm32& a, const APosNrm32& b, float thr) {
+    const float x = a.nx * b.nx, y = a.ny * b.ny, z = a.nz * b.nz;
+    const float d = x + y + z - thr, e = 6e-7f * (fabsf(x) + fabsf(y) + fabsf(z) + fabsf(thr)) + 1e-35f;
+    return d > e ? 1 : d < -e ? -1 : 0;  // NaN and infinities: 0
+}
+
+constexpr uint32_t kSharedMax = 16;  // corners of a group whose pairs are all looked at
+
+__global__ void smooth_shared_kernel(const APosNrm64* pn, const APosNrm32* pn32, const uint32_t* start,
+                                     const uint32_t* count, const uint32_t* member, uint64_t G, float thr,
+                                     uint8_t* shared, double* gsum) {
+    GRID_LOOP(g, G) {
+        const uint32_t n = count[g];
+        const uint32_t* m = member + start[g];
+        bool all = n != 0 && n <= kSharedMax;
+        for (uint32_t i = 0; all && i < n; i++) {
+            const APosNrm32 a = pn32[m[i]];
+            for (uint32_t k = i; all && k < n; k++) all = side_of(a, pn32[m[k]], thr) > 0;
+        }
+        shared[g] = all ? 1 : 0;
+        if (!all) continue;
+        V3d s = mv(0, 0, 0);
+        for (uint32_t k = 0; k < n; k++) s = vadd(s, nrm_of(pn, m[k]));
+        put3(gsum, g, vnormalize(s));
+    }
+}
+
+__global__ void smooth_threshold_kernel(const APosNrm64* pn, const APosNrm32* pn32, const uint32_t* gid,
+                                        const uint32_t* start, const uint32_t* count, const uint32_t* member,
+                                        uint64_t V, double threshold, const uint8_t* shared, double* out) {
     GRID_LOOP(c, V) {
-        const V3d normal = nrm_of(pn, c);
-        V3d result = mv(0, 0, 0);
         const uint32_t g = gid[c];
+        if (g != kNoGroup && shared[g]) continue;
+        V3d result = mv(0, 0, 0);
         if (g != kNoGroup) {
+            const V3d normal = nrm_of(pn, c);
+            const APosNrm32 n32 = pn32[c];
+            const float thr = (float)threshold;
             const uint32_t* m = member + start[g];
             for (uint32_t k = 0; k < count[g]; k++) {
+                const int side = side_of(pn32[m[k]], n32, thr);
+                if (side < 0) continue;
                 const V3d x = nrm_of(pn, m[k]);
-                if (vdot(x, normal) >= threshold) result = vadd(result, x);
+                if (side > 0 || vdot(x, normal) >= threshold) result = vadd(result, x);
             }
         }
         put3(out, c, vnormalize(result));
@@ -200,9 +242,13 @@ __global__ void smooth_assign_kernel(const uint32_t* gid, const double* gsum, ui
     }
 }
 
-__global__ void set_normals_kernel(const double* nrm, uint64_t V, APosNrm64* pn64, APosNrm32* pn32) {
+// The corners' new normals: their group's where `shared` says so (null: none),
+// else their own in nrm.
+__global__ void set_normals_kernel(const double* nrm, const uint32_t* gid, const uint8_t* shared, const double* gsum,
+                                   uint64_t V, APosNrm64* pn64, APosNrm32* pn32) {
     GRID_LOOP(c, V) {
-        const V3d n = get3(nrm, c);
+        const uint32_t g = shared ? gid[c] : kNoGroup;
+        const V3d n = g != kNoGroup && shared[g] ? get3(gsum, g) : get3(nrm, c);
         pn64[c].nx = n.x;
         pn64[c].ny = n.y;
         pn64[c].nz = n.z;
@@ -225,8 +271,25 @@ __device__ __forceinline__ bool has_edge(const uint32_t* gid, uint64_t t, uint32
            (g2 == ga && g0 == gb) || (g2 == gb && g0 == ga);
 }
 
-__global__ void sharp_flag_kernel(const APosNrm64* pn, const uint32_t* gid, const uint32_t* start,
-                                  const uint32_t* count, const uint32_t* member, uint64_t T, double angle,
+// Triangle.Normal of every triangle, once instead of for each of its edges.
+__global__ void sharp_normals_kernel(const APosNrm64* pn, uint64_t T, double* nrm) {
+    GRID_LOOP(t, T) put3(nrm, t, face_normal(pos_of(pn, 3 * t), pos_of(pn, 3 * t + 1), pos_of(pn, 3 * t + 2)));
+}
+
+// Whether acos(x) > angle (mesh.go:281), c = cos(angle) for an angle in [0, pi]
+// and NaN otherwise: acos falls by at least as much as x rises, so a cosine
+// 1e-10 off c on [-1, 1] decides it far beyond acos's error of an ulp or two,
+// and acos itself runs only on what is nearer, out of its domain or NaN.
+__device__ __forceinline__ bool sharper(double x, double angle, double c) {
+    if (x >= -1.0 && x < c - 1e-10) return true;
+    if (x <= 1.0 && x > c + 1e-10) return false;
+    return acos(x) > angle;
+}
+
+// FP64-bound before: two face normals and an arc cosine for each of 983,040
+// edges, 383 us; one normal per triangle and a dot product per edge take 55 us (kernels).
+__global__ void sharp_flag_kernel(const double* fn, const uint32_t* gid, const uint32_t* start,
+                                  const uint32_t* count, const uint32_t* member, uint64_t T, double angle, double c,
                                   uint32_t* flag) {
     GRID_LOOP(o, 3 * T) {
         const uint64_t t = o / 3;
@@ -244,11 +307,7 @@ __global__ void sharp_flag_kernel(const APosNrm64* pn, const uint32_t* gid, cons
                     break;
                 }
             }
-            if (u >= 0) {
-                const V3d nt = face_normal(pos_of(pn, 3 * t), pos_of(pn, 3 * t + 1), pos_of(pn, 3 * t + 2));
-                const V3d nu = face_normal(pos_of(pn, 3 * u), pos_of(pn, 3 * u + 1), pos_of(pn, 3 * u + 2));
-                if (acos(vdot(nt, nu)) > angle) f = 1;
-            }
+            if (u >= 0 && sharper(vdot(get3(fn, t), get3(fn, (uint64_t)u)), angle, c)) f = 1;
         }
         flag[o] = f;
     }
@@ -595,11 +654,16 @@ int fgc_mesh_smooth_normals_threshold(fgc_mesh* m, double radians) {
     if (W.rc) return W.rc;
     const double threshold = std::cos(radians);
     Groups Gr;
-    TempBuf<double> out;
-    if (!build_groups(W, m, V, Gr) || !W.ok(out.ensure(3 * V, W.s), "alloc normals")) return W.rc;
-    smooth_threshold_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, V,
-                                                         threshold, out.p);
-    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, V, m->pn64.p, m->pn32.p);
+    TempBuf<double> out, gsum;
+    TempBuf<uint8_t> shared;
+    if (!build_groups(W, m, V, Gr) || !W.ok(out.ensure(3 * V, W.s), "alloc normals") ||
+        !W.ok(gsum.ensure(3 * Gr.G, W.s), "alloc sums") || !W.ok(shared.ensure(Gr.G, W.s), "alloc flags"))
+        return W.rc;
+    smooth_shared_kernel<<<W.grid(Gr.G), 256, 0, W.s>>>(m->pn64.p, m->pn32.p, Gr.start.p, Gr.count.p, Gr.member.p, Gr.G,
+                                                         (float)threshold, shared.p, gsum.p);
+    smooth_threshold_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, m->pn32.p, Gr.gid.p, Gr.start.p, Gr.count.p,
+                                                         Gr.member.p, V, threshold, shared.p, out.p);
+    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, Gr.gid.p, shared.p, gsum.p, V, m->pn64.p, m->pn32.p);
     W.ok(cudaGetLastError(), "smoothing kernels");
     W.ok(cudaStreamSynchronize(W.s), "smoothing");
     return W.rc;
@@ -613,7 +677,7 @@ int fgc_mesh_smooth_normals(fgc_mesh* m) {
     if (W.rc) return W.rc;
     TempBuf<double> out;
     if (!W.ok(out.ensure(3 * V, W.s), "alloc normals") || !smooth_normals_into(W, m, out.p)) return W.rc;
-    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, V, m->pn64.p, m->pn32.p);
+    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, nullptr, nullptr, nullptr, V, m->pn64.p, m->pn32.p);
     W.ok(cudaGetLastError(), "smoothing kernels");
     W.ok(cudaStreamSynchronize(W.s), "smoothing");
     return W.rc;
@@ -629,11 +693,13 @@ int fgc_mesh_sharp_edges(const fgc_mesh* m, double angle_threshold, fgc_mesh** o
     if (T == 0) return line_mesh(W, nullptr, 0, out);
     Groups Gr;
     TempBuf<uint32_t> flag, pos;
-    TempBuf<double> lines;
-    if (!build_groups(W, m, 3 * T, Gr) || !W.ok(flag.ensure(E, W.s), "alloc flags") || !W.ok(pos.ensure(E, W.s), "alloc flags"))
+    TempBuf<double> lines, fn;
+    if (!build_groups(W, m, 3 * T, Gr) || !W.ok(fn.ensure(3 * T, W.s), "alloc normals") || !W.ok(flag.ensure(E, W.s), "alloc flags") || !W.ok(pos.ensure(E, W.s), "alloc flags"))
         return W.rc;
-    sharp_flag_kernel<<<W.grid(E), 256, 0, W.s>>>(m->pn64.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, T,
-                                                   angle_threshold, flag.p);
+    const double c = angle_threshold >= 0 && angle_threshold <= 3.141592653589793 ? std::cos(angle_threshold) : NAN;
+    sharp_normals_kernel<<<W.grid(T), 256, 0, W.s>>>(m->pn64.p, T, fn.p);
+    sharp_flag_kernel<<<W.grid(E), 256, 0, W.s>>>(fn.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, T,
+                                                   angle_threshold, c, flag.p);
     uint64_t n = 0;
     if (!W.ok(cudaGetLastError(), "edge kernel") || !scan_u32(W, flag.p, pos.p, E, &n)) return W.rc;
     if (!W.ok(lines.ensure(6 * std::max<uint64_t>(n, 1), W.s), "alloc lines")) return W.rc;
