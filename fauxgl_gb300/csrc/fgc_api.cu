@@ -354,15 +354,16 @@ int mesh_weld_attrs(fgc_mesh* m, cudaStream_t s, int sms, const double* cp, cons
         uint64_t tsize = 1;
         while (tsize < 2 * V) tsize <<= 1;
         const uint64_t scan_tiles = (V + 2047) / 2048;
+        // words after the scan tiles: status, ticket; unusual coordinate seen
         if (!step(table.ensure(2 * tsize, s), "alloc weld table") || !step(slot_of.ensure(V, s), "alloc weld") ||
             !step(flag.ensure(V, s), "alloc weld") || !step(uid.ensure(V, s), "alloc weld") ||
-            !step(tiles.ensure(scan_tiles + 2, s), "alloc scan"))
+            !step(tiles.ensure(scan_tiles + 3, s), "alloc scan"))
             break;
         uint32_t* minc = table.p + tsize;
         unsigned int* st = (unsigned int*)(tiles.p + scan_tiles + 1);
         if (!step(cudaMemsetAsync(table.p, 0xFF, 2 * tsize * 4, s), "init table")) break;
-        if (!step(cudaMemsetAsync(tiles.p, 0, (scan_tiles + 2) * 8, s), "zero scan")) break;
-        weld_insert_kernel<<<grid, 256, 0, s>>>(cp, V, table.p, tsize - 1, slot_of.p, minc, st);
+        if (!step(cudaMemsetAsync(tiles.p, 0, (scan_tiles + 3) * 8, s), "zero scan")) break;
+        weld_insert_kernel<<<grid, 256, 0, s>>>(cp, V, table.p, tsize - 1, slot_of.p, minc, st, st + 2);
         weld_flag_kernel<<<grid, 256, 0, s>>>(slot_of.p, minc, V, flag.p);
         ScanParams sp;
         sp.n_dev = nullptr;
@@ -372,14 +373,15 @@ int mesh_weld_attrs(fgc_mesh* m, cudaStream_t s, int sms, const double* cp, cons
         sp.lb = Lookback{tiles.p + 1, st + 1, st, tiles.p};
         scan_u32_kernel<<<(unsigned)scan_tiles, 256, 0, s>>>(sp);
         if (!step(cudaGetLastError(), "weld kernels")) break;
-        unsigned long long h_tot[2] = {0, 0};
+        unsigned long long h_tot[3] = {0, 0, 0};
         if (!step(cudaMemcpyAsync(&h_tot[0], tiles.p, 8, cudaMemcpyDeviceToHost, s), "read unique count")) break;
-        if (!step(cudaMemcpyAsync(&h_tot[1], st, 4, cudaMemcpyDeviceToHost, s), "read status")) break;
+        if (!step(cudaMemcpyAsync(&h_tot[1], st, 16, cudaMemcpyDeviceToHost, s), "read status")) break;
         if (!step(cudaStreamSynchronize(s), "weld")) break;
         if ((unsigned int)h_tot[1] != 0) {
             rc = fail(FGC_ERR_DEVICE_LIMIT, "mesh weld failed");
             break;
         }
+        m->plain_positions = (unsigned int)h_tot[2] == 0;
         m->nuniq = h_tot[0];
         if (!step(m->ux.ensure(m->nuniq + 1, s), "alloc unique") || !step(m->uy.ensure(m->nuniq + 1, s), "alloc unique") ||
             !step(m->uz.ensure(m->nuniq + 1, s), "alloc unique") || !step(m->corner_uniq.ensure(V, s), "alloc index"))

@@ -204,6 +204,7 @@ struct fgc_mesh {
     fgc::MeshBuf<double> tex64, col64;
     fgc::MeshBuf<float> tex32, col32;
     bool has_tex = false, has_col = false;
+    bool plain_positions = false;  // no coordinate is -0 or NaN: equal positions have equal bits
 
     fgc::MeshView view() const {
         fgc::MeshView v;

@@ -304,7 +304,7 @@ __global__ void downsample_kernel(const uint32_t* src, int32_t w, int32_t h, int
 __global__ void depth_minmax_kernel(const double* d, uint64_t n, unsigned long long* lohi);
 __global__ void depth_image_kernel(const double* d, uint64_t n, const unsigned long long* lohi, uint16_t* out);
 __global__ void weld_insert_kernel(const double* cp, uint64_t n, uint32_t* table, uint64_t tmask,
-                                   uint32_t* slot_of, uint32_t* minc, unsigned int* status);
+                                   uint32_t* slot_of, uint32_t* minc, unsigned int* status, unsigned int* unusual);
 __global__ void weld_flag_kernel(const uint32_t* slot_of, const uint32_t* minc, uint64_t n, uint32_t* flag);
 __global__ void weld_emit_kernel(const double* cp, const uint32_t* slot_of, const uint32_t* minc,
                                  const uint32_t* uid, uint64_t n, double* ux, double* uy, double* uz,

@@ -14,7 +14,8 @@
 // corners are grouped by the bit pattern of position + 0.0 through the weld's
 // hash table; NaN positions get no group. A group lists its corners in corner
 // order -- the order of the reference's appends -- so every sum below adds in
-// the reference's order and gives its bits. Vector arithmetic follows
+// the reference's order and gives its bits. Where the weld saw no coordinate
+// that is -0 or NaN its own numbering of the positions is such a grouping. Vector arithmetic follows
 // vector.go left to right (the library is built without contraction).
 #include <cmath>
 #include <cstdlib>
@@ -126,6 +127,10 @@ __global__ void group_ids_kernel(const uint32_t* slot_of, const uint32_t* minc, 
     }
 }
 
+__global__ void group_count_kernel(const uint32_t* gid, uint64_t V, uint32_t* count) {
+    GRID_LOOP(c, V) atomicAdd(&count[gid[c]], 1u);
+}
+
 __global__ void group_fill_kernel(const uint32_t* gid, const uint32_t* start, uint32_t* cursor, uint64_t V,
                                   uint32_t* member) {
     GRID_LOOP(c, V) {
@@ -165,7 +170,8 @@ __global__ void group_sort_kernel(const uint32_t* start, const uint32_t* count, 
 // product reaches the threshold is decided in FP32 where it is further from
 // it than FP32 can be off (side_of); and where every pair of a group's normals
 // reaches it -- a smooth place -- all its corners have the same sum, formed
-// once (smooth_shared_kernel). SMOOTH_AFTER us for both.
+// once (smooth_shared_kernel). 100 us for both on a displaced
+// sphere of 327,680 triangles, where half the places are smooth.
 
 // +1: the FP64 dot product of the normals behind a and b is at least thr, -1:
 // below it, 0: too near to tell. The FP32 dot product of rounded components is
@@ -462,34 +468,46 @@ bool scan_u32(Work& W, const uint32_t* in, uint32_t* out, uint64_t n, uint64_t* 
 
 // Groups of the first V corners of a mesh by position (Go map keys).
 struct Groups {
-    TempBuf<uint32_t> gid, start, count, member;
+    TempBuf<uint32_t> own_gid, start, count, member;
+    const uint32_t* gid = nullptr;  // group of each corner: own_gid, or the mesh's unique-position index
     uint64_t G = 0;  // group slots (some may be empty)
 };
 
+bool fill_groups(Work& W, uint64_t V, Groups& Gr);
+
 bool build_groups(Work& W, const fgc_mesh* m, uint64_t V, Groups& Gr) {
+    if (m->plain_positions) {
+        // hashing the positions again took 55 of the 100 us of grouping
+        // 983,040 corners, and a wait for the host
+        Gr.gid = m->corner_uniq.p;
+        Gr.G = m->nuniq;
+        if (!W.ok(Gr.count.ensure(Gr.G, W.s), "alloc groups") ||
+            !W.ok(cudaMemsetAsync(Gr.count.p, 0, Gr.G * 4, W.s), "zero counts"))
+            return false;
+        group_count_kernel<<<W.grid(V), 256, 0, W.s>>>(Gr.gid, V, Gr.count.p);
+        return W.ok(cudaGetLastError(), "group kernels") && fill_groups(W, V, Gr);
+    }
     TempBuf<double> key;
     TempBuf<uint8_t> nanf;
-    TempBuf<uint32_t> table, slot_of, flag, uid, cursor;  // table: hash slots, then each slot's first corner
+    TempBuf<uint32_t> table, slot_of, flag, uid;  // table: hash slots, then each slot's first corner
     TempBuf<unsigned int> st;
     uint64_t tsize = 1;
     while (tsize < 2 * V) tsize <<= 1;
     if (!W.ok(key.ensure(3 * V, W.s), "alloc keys") || !W.ok(nanf.ensure(V, W.s), "alloc keys") ||
         !W.ok(table.ensure(2 * tsize, W.s), "alloc table") ||
         !W.ok(slot_of.ensure(V, W.s), "alloc groups") || !W.ok(flag.ensure(V, W.s), "alloc groups") ||
-        !W.ok(uid.ensure(V, W.s), "alloc groups") || !W.ok(cursor.ensure(V, W.s), "alloc groups") ||
-        !W.ok(Gr.gid.ensure(V, W.s), "alloc groups") || !W.ok(Gr.start.ensure(V, W.s), "alloc groups") ||
-        !W.ok(Gr.count.ensure(V, W.s), "alloc groups") || !W.ok(Gr.member.ensure(V, W.s), "alloc groups") ||
+        !W.ok(uid.ensure(V, W.s), "alloc groups") || !W.ok(Gr.own_gid.ensure(V, W.s), "alloc groups") ||
+        !W.ok(Gr.count.ensure(V, W.s), "alloc groups") ||
         !W.ok(st.ensure(1, W.s), "alloc status"))
         return false;
     const int grid = W.grid(V);
     uint32_t* const minc = table.p + tsize;
     if (!W.ok(cudaMemsetAsync(table.p, 0xFF, 2 * tsize * 4, W.s), "init table") ||
         !W.ok(cudaMemsetAsync(st.p, 0, 4, W.s), "zero status") ||
-        !W.ok(cudaMemsetAsync(Gr.count.p, 0, V * 4, W.s), "zero counts") ||
-        !W.ok(cudaMemsetAsync(cursor.p, 0, V * 4, W.s), "zero cursors"))
+        !W.ok(cudaMemsetAsync(Gr.count.p, 0, V * 4, W.s), "zero counts"))
         return false;
     group_keys_kernel<<<grid, 256, 0, W.s>>>(m->pn64.p, V, key.p, nanf.p);
-    weld_insert_kernel<<<grid, 256, 0, W.s>>>(key.p, V, table.p, tsize - 1, slot_of.p, minc, st.p);
+    weld_insert_kernel<<<grid, 256, 0, W.s>>>(key.p, V, table.p, tsize - 1, slot_of.p, minc, st.p, nullptr);
     weld_flag_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc, V, flag.p);
     if (!W.ok(cudaGetLastError(), "group kernels")) return false;
     uint64_t nrep = 0;
@@ -503,10 +521,22 @@ bool build_groups(Work& W, const fgc_mesh* m, uint64_t V, Groups& Gr) {
         return false;
     }
     Gr.G = nrep;
-    group_ids_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc, uid.p, nanf.p, V, Gr.gid.p, Gr.count.p);
+    Gr.gid = Gr.own_gid.p;
+    group_ids_kernel<<<grid, 256, 0, W.s>>>(slot_of.p, minc, uid.p, nanf.p, V, Gr.own_gid.p, Gr.count.p);
+    return W.ok(cudaGetLastError(), "group kernels") && fill_groups(W, V, Gr);
+}
+
+// The members of each group, in corner order, from the corners' groups and
+// the groups' sizes.
+bool fill_groups(Work& W, uint64_t V, Groups& Gr) {
+    TempBuf<uint32_t> cursor;
     uint64_t total = 0;
-    if (!W.ok(cudaGetLastError(), "group kernels") || !scan_u32(W, Gr.count.p, Gr.start.p, Gr.G, &total)) return false;
-    group_fill_kernel<<<grid, 256, 0, W.s>>>(Gr.gid.p, Gr.start.p, cursor.p, V, Gr.member.p);
+    if (!W.ok(cursor.ensure(Gr.G, W.s), "alloc groups") || !W.ok(Gr.start.ensure(Gr.G, W.s), "alloc groups") ||
+        !W.ok(Gr.member.ensure(V, W.s), "alloc groups") ||
+        !W.ok(cudaMemsetAsync(cursor.p, 0, Gr.G * 4, W.s), "zero cursors") ||
+        !scan_u32(W, Gr.count.p, Gr.start.p, Gr.G, &total))
+        return false;
+    group_fill_kernel<<<W.grid(V), 256, 0, W.s>>>(Gr.gid, Gr.start.p, cursor.p, V, Gr.member.p);
     group_sort_kernel<<<W.grid(Gr.G), 256, 0, W.s>>>(Gr.start.p, Gr.count.p, Gr.G, Gr.member.p);
     return W.ok(cudaGetLastError(), "group kernels");
 }
@@ -519,7 +549,7 @@ bool smooth_normals_into(Work& W, const fgc_mesh* m, double* out) {
     TempBuf<double> gsum;
     if (!W.ok(gsum.ensure(3 * std::max<uint64_t>(Gr.G, 1), W.s), "alloc sums")) return false;
     smooth_sum_kernel<<<W.grid(Gr.G), 256, 0, W.s>>>(m->pn64.p, Gr.start.p, Gr.count.p, Gr.member.p, Gr.G, gsum.p);
-    smooth_assign_kernel<<<W.grid(V), 256, 0, W.s>>>(Gr.gid.p, gsum.p, V, out);
+    smooth_assign_kernel<<<W.grid(V), 256, 0, W.s>>>(Gr.gid, gsum.p, V, out);
     return W.ok(cudaGetLastError(), "smoothing kernels");
 }
 
@@ -661,9 +691,9 @@ int fgc_mesh_smooth_normals_threshold(fgc_mesh* m, double radians) {
         return W.rc;
     smooth_shared_kernel<<<W.grid(Gr.G), 256, 0, W.s>>>(m->pn64.p, m->pn32.p, Gr.start.p, Gr.count.p, Gr.member.p, Gr.G,
                                                          (float)threshold, shared.p, gsum.p);
-    smooth_threshold_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, m->pn32.p, Gr.gid.p, Gr.start.p, Gr.count.p,
+    smooth_threshold_kernel<<<W.grid(V), 256, 0, W.s>>>(m->pn64.p, m->pn32.p, Gr.gid, Gr.start.p, Gr.count.p,
                                                          Gr.member.p, V, threshold, shared.p, out.p);
-    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, Gr.gid.p, shared.p, gsum.p, V, m->pn64.p, m->pn32.p);
+    set_normals_kernel<<<W.grid(V), 256, 0, W.s>>>(out.p, Gr.gid, shared.p, gsum.p, V, m->pn64.p, m->pn32.p);
     W.ok(cudaGetLastError(), "smoothing kernels");
     W.ok(cudaStreamSynchronize(W.s), "smoothing");
     return W.rc;
@@ -698,7 +728,7 @@ int fgc_mesh_sharp_edges(const fgc_mesh* m, double angle_threshold, fgc_mesh** o
         return W.rc;
     const double c = angle_threshold >= 0 && angle_threshold <= 3.141592653589793 ? std::cos(angle_threshold) : NAN;
     sharp_normals_kernel<<<W.grid(T), 256, 0, W.s>>>(m->pn64.p, T, fn.p);
-    sharp_flag_kernel<<<W.grid(E), 256, 0, W.s>>>(fn.p, Gr.gid.p, Gr.start.p, Gr.count.p, Gr.member.p, T,
+    sharp_flag_kernel<<<W.grid(E), 256, 0, W.s>>>(fn.p, Gr.gid, Gr.start.p, Gr.count.p, Gr.member.p, T,
                                                    angle_threshold, c, flag.p);
     uint64_t n = 0;
     if (!W.ok(cudaGetLastError(), "edge kernel") || !scan_u32(W, flag.p, pos.p, E, &n)) return W.rc;

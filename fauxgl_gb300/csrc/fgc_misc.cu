@@ -112,12 +112,18 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
+__device__ __forceinline__ bool odd_coordinate(long long b) {
+    return b == (long long)0x8000000000000000ull || (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+
 __global__ void weld_insert_kernel(const double* cp, uint64_t n, uint32_t* table, uint64_t tmask, uint32_t* slot_of,
-                                   uint32_t* minc, unsigned int* status) {
+                                   uint32_t* minc, unsigned int* status, unsigned int* unusual) {
     for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
         const long long bx = __double_as_longlong(cp[3 * c]);
         const long long by = __double_as_longlong(cp[3 * c + 1]);
         const long long bz = __double_as_longlong(cp[3 * c + 2]);
+        // -0 or NaN: the position's bits are not its identity as a map key
+        if (unusual && (odd_coordinate(bx) || odd_coordinate(by) || odd_coordinate(bz))) *unusual = 1;
         uint64_t h = mix64((unsigned long long)bx ^ mix64((unsigned long long)by ^ mix64((unsigned long long)bz))) & tmask;
         uint32_t slot = 0xFFFFFFFFu;
         for (uint64_t probe = 0; probe <= tmask; probe++) {
