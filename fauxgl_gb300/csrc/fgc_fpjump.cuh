@@ -100,56 +100,48 @@ FGC_HD double repeat_add(double s, double a, uint64_t k) {
         return k ? fj_add(s, a) : s;
     }
     const int ea = (int)((ab >> 52) & 0x7ff);
+    const int el = ea ? ea : 1;  // exponent of a's last place
     const uint64_t Ma = (ab & kFrac) | (ea ? kHidden : 0);
     while (k > 0) {
         s = fj_add(s, a);  // a real step: enters the binade the model then covers
         k--;
         if (k == 0) break;
         const uint64_t sb = fj_bits(s);
-        if ((sb & kExp) == kExp) return s;  // infinite or NaN: fixed from here
         const int es = (int)((sb >> 52) & 0x7ff);
-        if (es == 0) continue;              // zero or subnormal: plain steps
-        if (ea >= es) continue;             // |a| not below the binade: plain steps
+        const int sh = es - el;             // a/u = Ma / 2^sh
+        // infinite or NaN: fixed from here; |a| < u/2: t + a rounds back to t
+        if (es == 0x7ff || (sh >= 54 && ea < es && (((sb ^ ab) & kSign) == 0 || (sb & kFrac) > 1))) return s;
+        // zero, subnormal, or |a| not below the binade: plain steps
+        if (es == 0 || ea >= es || sh <= 0 || sh >= 54) continue;
         // work on |t|: it grows when t and a have the same sign
         const bool grow = ((sb ^ ab) & kSign) == 0;
-        uint64_t m = (sb & kFrac) | kHidden;  // |t| / u, in [2^52, 2^53)
-        // shrinking from the binade's first value leaves it (finer spacing
-        // below): plain steps
-        if (!grow && m <= kHidden + 1) continue;
-        const int sh = es - (ea ? ea : 1);  // a/u = Ma / 2^sh
-        if (sh <= 0) continue;              // (smallest binade, subnormal a)
-        if (sh >= 54) return s;             // |a| < u/2: t + a rounds back to t
-        const uint64_t q = Ma >> sh;
-        const uint64_t rem = Ma & ((1ull << sh) - 1);
+        const uint64_t m = (sb & kFrac) | kHidden;  // |t| / u, in [2^52, 2^53)
+        // |t| changes by d = RN(a/u) (in units of u) per step
         const uint64_t half = 1ull << (sh - 1);
-        uint64_t d;                           // |t| changes by d (in units of u) per step
-        if (rem != half) {
-            d = q + (rem > half ? 1 : 0);
-        } else {
+        const uint64_t r = Ma + half;
+        uint64_t d = r >> sh;
+        const uint64_t q = Ma >> sh;
+        if ((r & (half + half - 1)) == 0) {
             // tie: the even neighbour. m + q and m - q have the parity of
             // m + q; once m is even (after one tie step) d is constant.
             if ((m & 1) != 0) continue;
-            d = q + (q & 1);
+            d &= ~1ull;
         }
-        if (d == 0) return s;               // t + a rounds back to t from here on
         // steps that keep every exact sum (before rounding) inside the
-        // binade, with one unit of margin at both ends
-        uint64_t avail;  // n steps fit when (n - 1) * d <= avail
-        if (grow) {
-            const uint64_t lim = kTop - 2;  // m_i + q <= 2^53 - 2
-            if (m + q > lim) continue;
-            avail = lim - m - q;
-        } else {
-            const uint64_t lim = kHidden + 1;  // m_i - q >= 2^52 + 1
-            if (m < q + lim) continue;
-            avail = m - q - lim;
-        }
+        // binade, with one unit of margin at both ends (shrinking from the
+        // binade's first value leaves it: finer spacing below): n steps fit
+        // when (n - 1) * d <= avail
+        const int64_t avail = (int64_t)(grow ? (kTop - 2) - m : m - (kHidden + 1)) - (int64_t)q;
+        if (!grow && m <= kHidden + 1) continue;
+        if (d == 0) return s;               // t + a rounds back to t from here on
+        if (avail < 0) continue;
         // all k remaining steps usually fit: only a jump that reaches the
         // binade's end needs the division
-        const uint64_t n = fj_mul_fits(k - 1, d, avail) ? k : (k <= (1u << 20) ? fj_div_small(avail, d) : avail / d) + 1;
-        m = grow ? m + n * d : m - n * d;
+        const uint64_t n = fj_mul_fits(k - 1, d, (uint64_t)avail)
+                               ? k : (k <= (1u << 20) ? fj_div_small((uint64_t)avail, d) : (uint64_t)avail / d) + 1;
+        const uint64_t nd = n * d;
         k -= n;
-        s = fj_double((sb & kSign) | ((uint64_t)es << 52) | (m - kHidden));
+        s = fj_double((sb & (kSign | kExp)) | ((grow ? m + nd : m - nd) & kFrac));
     }
     return s;
 }
