@@ -371,7 +371,7 @@ int mesh_weld_attrs(fgc_mesh* m, cudaStream_t s, int sms, const double* cp, cons
         sp.out = uid.p;
         sp.n = V;
         sp.lb = Lookback{tiles.p + 1, st + 1, st, tiles.p};
-        scan_u32_kernel<<<(unsigned)scan_tiles, 256, 0, s>>>(sp);
+        scan_u32_kernel<<<(unsigned)scan_tiles, 256, 0, s>>>(sp, sp, (uint32_t)scan_tiles);
         if (!step(cudaGetLastError(), "weld kernels")) break;
         unsigned long long h_tot[3] = {0, 0, 0};
         if (!step(cudaMemcpyAsync(&h_tot[0], tiles.p, 8, cudaMemcpyDeviceToHost, s), "read unique count")) break;

@@ -287,7 +287,7 @@ __global__ void clip_piece_kernel(GeomParams P);
 __global__ void clip_lines_kernel(GeomParams P);
 
 __global__ void bin_count_kernel(BinParams P);
-__global__ void scan_u32_kernel(ScanParams P);
+__global__ void scan_u32_kernel(ScanParams A, ScanParams B, uint32_t first);
 __global__ void bin_scatter_kernel(BinParams P, int warps);
 __global__ void row_starts_kernel(RowStartParams P);
 

@@ -451,7 +451,7 @@ bool scan_u32(Work& W, const uint32_t* in, uint32_t* out, uint64_t n, uint64_t* 
     sp.out = out;
     sp.n = n;
     sp.lb = Lookback{tiles.p + 1, words.p, words.p + 1, tiles.p};
-    scan_u32_kernel<<<(unsigned)nt, 256, 0, W.s>>>(sp);
+    scan_u32_kernel<<<(unsigned)nt, 256, 0, W.s>>>(sp, sp, (uint32_t)nt);
     unsigned long long h[2] = {0, 0};
     if (!W.ok(cudaGetLastError(), "scan") ||
         !W.ok(cudaMemcpyAsync(&h[0], tiles.p, 8, cudaMemcpyDeviceToHost, W.s), "read scan total") ||

@@ -25,6 +25,7 @@ struct Lookback {
     unsigned long long* total;  // receives the grand total (written by the last block)
     uint32_t spin_limit = kSpinLimit;   // polls of an unpublished predecessor before giving up
     uint32_t withhold = 0xFFFFFFFFu;    // test hook: this logical block never publishes
+    uint32_t ntiles = 0;                // logical blocks; 0: every block of the grid is one
 };
 
 template <int BLOCK>
@@ -113,7 +114,7 @@ __device__ __forceinline__ uint64_t lookback_prefix(const Lookback& L, uint32_t 
                 atomicExch(&L.tiles[tile], (unsigned long long)(kFlagPre | ((excl + agg) & kValMask)));
         }
         if (lane == 0) {
-            if (tile == gridDim.x - 1 && L.total) *L.total = excl + agg;
+            if (tile == (L.ntiles ? L.ntiles : gridDim.x) - 1 && L.total) *L.total = excl + agg;
             *s_prefix = excl;
         }
     }
