@@ -672,6 +672,15 @@ __device__ FullVertex load_corner(const GeomParams& P, const ItemView& I, uint64
 // kernels run on a side stream: the first two beside the scan and the list
 // writer, the third (it needs the slots the list writer assigns) beside the
 // emission.
+//
+// Up to kClipSmall entries clip_poly_kernel gives each a warp, which also
+// makes the vertices. The steps are serial FP64 chains (a lone warp's FP64
+// instruction takes 64 cycles), 16 + 10 us however few the entries are, and
+// with the third longer than the rest of a small pass's setup; a lane per
+// vertex makes the first two 10 us together: setup of 54 entries (128x128)
+// 53 -> 43 us, of 575 (1280x720) 55 -> 44, of 1,259 (1600x900) 74 -> 70. Its
+// FP64 instructions have at most nine lanes at work, so that many entries are
+// cheaper packed: 2,419 (1080p) 145 us a thread each, 162 a warp each.
 __device__ __forceinline__ FullVertex clip_vertex(const FullVertex* tv, D3 p1, D3 p2, D3 p3, D4 q, uint32_t mask) {
     const D4 bw = barycentric(p1, p2, p3, d3(q.x, q.y, q.z));
     FullVertex v;
@@ -680,8 +689,72 @@ __device__ __forceinline__ FullVertex clip_vertex(const FullVertex* tv, D3 p1, D
     return v;
 }
 
+// Polygon vertex q (clip space) of clipped triangle elem, with its
+// interpolated attributes and NDC position.
+__device__ __forceinline__ ClipVert make_clip_vert(const GeomParams& P, const ItemView& I, uint32_t elem, D4 q) {
+    const uint32_t mask = I.attr_mask;
+    FullVertex tv[3];
+    for (int c = 0; c < 3; c++) tv[c] = load_corner(P, I, 3 * (uint64_t)elem + c);
+    if (mask & kAttrNrm) fix_normals(tv[0], tv[1], tv[2]);  // NewTriangle(v1, v2, v3)
+    const D3 p1 = d3(tv[0].out.x, tv[0].out.y, tv[0].out.z);
+    const D3 p2 = d3(tv[1].out.x, tv[1].out.y, tv[1].out.z);
+    const D3 p3 = d3(tv[2].out.x, tv[2].out.y, tv[2].out.z);
+    const FullVertex v = clip_vertex(tv, p1, p2, p3, q, mask);
+    const D3 nd = ndc_of(v.out);
+    return ClipVert{v.pos.x, v.pos.y, v.pos.z, v.nrm.x, v.nrm.y, v.nrm.z, v.tu, v.tv,
+                    v.col.x, v.col.y, v.col.z, v.col.w, v.out.x, v.out.y, v.out.z, v.out.w,
+                    nd.x, nd.y, nd.z};
+}
+
+// Entry e's polygon and vertices by one warp: lane j holds polygon vertex j, and
+// the places of a plane's output vertices follow from the ballots of crossing
+// edges and kept vertices.
+__device__ __forceinline__ void clip_entry_warp(const GeomParams& P, uint32_t e) {
+    constexpr int kPolyMax = 16;  // as the buffers of the form below
+    __shared__ D4 s_poly[kPolyMax];
+    const uint32_t lane = threadIdx.x, lt = (1u << lane) - 1u;
+    const ClipEntry ent = P.clip_list[e];
+    const ItemView& I = P.items[ent.item];
+    const VClip* vc = P.vclip + I.vbase;
+    D4 v = d4(0, 0, 0, 0);
+    if (lane < 3) {
+        const VClip o = vc[I.mesh.corner_uniq[3 * (uint64_t)ent.elem + lane]];
+        v = d4(o.x, o.y, o.z, o.w);
+    }
+    uint32_t np = 3;
+#pragma unroll 1
+    for (int k = 0; k < 6 && np > 0; k++) {
+        const bool f = lane < np && point_in_front(k, v);
+        const uint32_t fm = __ballot_sync(0xffffffffu, f);
+        if (fm == (1u << np) - 1u) continue;  // the plane leaves the polygon as it is
+        const int prev = lane == 0 ? (int)np - 1 : (int)lane - 1;
+        const D4 s = d4(__shfl_sync(0xffffffffu, v.x, prev), __shfl_sync(0xffffffffu, v.y, prev),
+                        __shfl_sync(0xffffffffu, v.z, prev), __shfl_sync(0xffffffffu, v.w, prev));
+        // the edge from the vertex before this one crosses the plane
+        const bool cross = lane < np && f != (((fm >> prev) & 1u) != 0);
+        const uint32_t cm = __ballot_sync(0xffffffffu, cross);
+        uint32_t at = (uint32_t)__popc(cm & lt) + (uint32_t)__popc(fm & lt);
+        if (cross) {
+            if (at < kPolyMax) s_poly[at] = intersect_segment(k, s, v);
+            at++;
+        }
+        if (f && at < kPolyMax) s_poly[at] = v;
+        __syncwarp();
+        np = min((uint32_t)__popc(cm) + (uint32_t)__popc(fm), (uint32_t)kPolyMax);
+        if (lane < np) v = s_poly[lane];
+        __syncwarp();
+    }
+    if (lane == 0) P.cpoly[e].n = np;
+    if (np >= 3 && lane < min(np, (uint32_t)kClipPoly))
+        P.cvert[(uint64_t)e * kClipPoly + lane] = make_clip_vert(P, I, ent.elem, v);
+}
+
 __global__ void __launch_bounds__(32) clip_poly_kernel(GeomParams P) {
     const uint32_t n = min(*P.clip_count, P.clip_cap);
+    if (n <= kClipSmall) {
+        for (uint32_t e = blockIdx.x; e < n; e += gridDim.x) clip_entry_warp(P, e);
+        return;
+    }
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const ClipEntry ent = P.clip_list[e];
         const ItemView& I = P.items[ent.item];
@@ -725,25 +798,15 @@ __global__ void __launch_bounds__(32) clip_poly_kernel(GeomParams P) {
 }
 
 __global__ void __launch_bounds__(64) clip_vert_kernel(GeomParams P) {
-    const uint64_t n = (uint64_t)min(*P.clip_count, P.clip_cap) * kClipPoly;
+    const uint32_t entries = min(*P.clip_count, P.clip_cap);
+    if (entries <= kClipSmall) return;  // clip_poly_kernel made the vertices
+    const uint64_t n = (uint64_t)entries * kClipPoly;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t e = (uint32_t)(i / kClipPoly), j = (uint32_t)(i % kClipPoly);
         const uint32_t np = P.cpoly[e].n;
         if (np < 3 || j >= np) continue;  // no fan, or a vertex the fan does not read
         const ClipEntry ent = P.clip_list[e];
-        const ItemView& I = P.items[ent.item];
-        const uint32_t mask = I.attr_mask;
-        FullVertex tv[3];
-        for (int c = 0; c < 3; c++) tv[c] = load_corner(P, I, 3 * (uint64_t)ent.elem + c);
-        if (mask & kAttrNrm) fix_normals(tv[0], tv[1], tv[2]);  // NewTriangle(v1, v2, v3)
-        const D3 p1 = d3(tv[0].out.x, tv[0].out.y, tv[0].out.z);
-        const D3 p2 = d3(tv[1].out.x, tv[1].out.y, tv[1].out.z);
-        const D3 p3 = d3(tv[2].out.x, tv[2].out.y, tv[2].out.z);
-        const FullVertex v = clip_vertex(tv, p1, p2, p3, P.cpoly[e].v[j], mask);
-        const D3 nd = ndc_of(v.out);
-        P.cvert[i] = ClipVert{v.pos.x, v.pos.y, v.pos.z, v.nrm.x, v.nrm.y, v.nrm.z, v.tu, v.tv,
-                              v.col.x, v.col.y, v.col.z, v.col.w, v.out.x, v.out.y, v.out.z, v.out.w,
-                              nd.x, nd.y, nd.z};
+        P.cvert[i] = make_clip_vert(P, P.items[ent.item], (uint32_t)ent.elem, P.cpoly[e].v[j]);
     }
 }
 

@@ -156,6 +156,8 @@ struct GeomParams {
     uint32_t* cidx;             // per element of a setup tile: its clip_list entry, for a clipped triangle
     unsigned long long* tsum;   // per setup tile: slots << 31 | work items, then their exclusive prefix
 };
+// Clip entries a pass may have for each to get a warp of its own (fgc_geometry.cu says why).
+constexpr uint32_t kClipSmall = 2048;
 constexpr int kSetupTile = 256;  // threads of a setup tile
 constexpr int kSetupPer = 2;     // consecutive elements per thread
 

@@ -558,8 +558,9 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
             FGC_CUDA(cudaEventRecord(S.ev_fork, stream));
             FGC_CUDA(cudaStreamWaitEvent(S.side, S.ev_fork, 0));
             // one warp per block: a few thousand clip entries still spread
-            // over every SM's FP64 pipes
-            clip_poly_kernel<<<grid_for(S.clip_cap, 32, D.sms * 8), 32, 0, S.side>>>(gp);
+            // over every SM's FP64 pipes, and kClipSmall of them have a warp
+            // each
+            clip_poly_kernel<<<D.sms * 16, 32, 0, S.side>>>(gp);
             clip_vert_kernel<<<grid_for((uint64_t)S.clip_cap * kClipPoly, 64, D.sms * 8), 64, 0, S.side>>>(gp);
             FGC_CUDA(cudaGetLastError());
             rec.launches += 2;
