@@ -21,8 +21,11 @@ struct fgc_batch {
     bool use_graph = false;
     cudaGraphExec_t exec = nullptr;
     Submission sub;
+    cudaStream_t copy = nullptr;    // read-backs beside a later pass
+    cudaEvent_t copied = nullptr;
     struct ReadBack {
         fgc_context* ctx;
+        uint32_t item;
         uint8_t* dst;
         int32_t scale;
         size_t ds_off;  // offset in ds (scaled read-backs)
@@ -38,24 +41,84 @@ struct fgc_batch {
 
 namespace {
 
-// Queue the read-backs of a submission (after its passes).
-int enqueue_reads(fgc_batch* b) {
+// Copying (us) from which a submission's read-backs are split, and the share
+// of its pixels in the first pass. A second pass costs 0.1 to 0.16 ms of small
+// kernels: 24 frames of 64x64 (240 us of copies) 475 us in one pass, 490 in
+// two; 40 of 128x128 (400 us) 795 and 757. The last quarter's copies stay
+// behind the draws; with half in the first pass 48 mixed thumbnails take 3.52
+// ms, with 7/10 3.28, 3/4 3.23, 8/10 3.29, 7/8 3.45.
+constexpr double kReadCutMin = 360;
+constexpr uint64_t kReadCutNum = 3, kReadCutDen = 4;
+
+// Queue the read-backs of items [lo, hi) on stream s.
+int enqueue_reads(fgc_batch* b, uint32_t lo, uint32_t hi, cudaStream_t s) {
     const DevLimits* D = nullptr;
     int rc = dev_limits(b->device, &D);
     if (rc) return rc;
+    // every downsample before the first copy: a copy to pageable memory holds
+    // this thread, and a raster kernel that has begun leaves them no room
     for (const fgc_batch::ReadBack& r : b->reads) {
+        if (r.item < lo || r.item >= hi || r.scale <= 1) continue;
         const fgc_context* c = r.ctx;
-        if (r.scale <= 1) {
-            FGC_CUDA(cudaMemcpyAsync(r.dst, c->color.p, (size_t)c->N * 4, cudaMemcpyDeviceToHost, b->stream));
-            continue;
-        }
         const uint64_t n = (uint64_t)(c->W / r.scale) * (uint64_t)(c->H / r.scale);
-        uint32_t* dst = b->ds.p + r.ds_off;
-        downsample_kernel<<<grid_for(n, 256, D->sms * 8), 256, 0, b->stream>>>(c->color.p, c->W, c->H, r.scale, dst);
+        downsample_kernel<<<grid_for(n, 256, D->sms * 8), 256, 0, s>>>(c->color.p, c->W, c->H, r.scale,
+                                                                       b->ds.p + r.ds_off);
         FGC_CUDA(cudaGetLastError());
-        FGC_CUDA(cudaMemcpyAsync(r.dst, dst, n * 4, cudaMemcpyDeviceToHost, b->stream));
+    }
+    for (const fgc_batch::ReadBack& r : b->reads) {
+        if (r.item < lo || r.item >= hi) continue;
+        const fgc_context* c = r.ctx;
+        const uint64_t n = (uint64_t)(c->W / r.scale) * (uint64_t)(c->H / r.scale);
+        const uint32_t* src = r.scale > 1 ? b->ds.p + r.ds_off : c->color.p;
+        FGC_CUDA(cudaMemcpyAsync(r.dst, src, n * 4, cudaMemcpyDeviceToHost, s));
     }
     return FGC_OK;
+}
+
+// Queue the read-backs of a submission (after its passes); those of the items
+// before a cut run beside the passes after it.
+int enqueue_all_reads(fgc_batch* b) {
+    const uint32_t n = (uint32_t)b->sub.items.size(), cut = b->sub.cut;
+    if (cut) {
+        FGC_CUDA(cudaStreamWaitEvent(b->copy, b->sub.at_cut, 0));
+        int rc = enqueue_reads(b, 0, cut, b->copy);
+        if (rc) return rc;
+        FGC_CUDA(cudaEventRecord(b->copied, b->copy));
+    }
+    int rc = enqueue_reads(b, cut, n, b->stream);
+    if (rc) return rc;
+    if (cut) FGC_CUDA(cudaStreamWaitEvent(b->stream, b->copied, 0));
+    return FGC_OK;
+}
+
+// The item of a submission that begins a second pass, or 0: copying the frames
+// of the first pass then runs beside the second. Read back one after the other
+// behind all draws, 48 frames of 85 MB took 1.05 ms of 3.74 (190 GB/s over the
+// link and 10 us a copy); so they take 3.23 ms, and 20 frames drawn at four
+// samples a pixel 5.09 ms instead of 5.34.
+uint32_t read_cut(const fgc_batch* b) {
+    const std::vector<PassItem>& items = b->sub.items;
+    if (b->use_graph || b->reads.empty()) return 0;
+    // a frame drawn more than once is read after its last draw, and passes of
+    // their own follow from it or from a change of precision
+    std::vector<const fgc_context*> targets;
+    for (const PassItem& p : items) {
+        if (p.sv.precision != items[0].sv.precision) return 0;
+        targets.push_back(p.ctx);
+    }
+    std::sort(targets.begin(), targets.end());
+    if (std::adjacent_find(targets.begin(), targets.end()) != targets.end()) return 0;
+    double us = 0;
+    for (const fgc_batch::ReadBack& r : b->reads)
+        us += 10.0 + (double)r.ctx->N * 4 / ((double)r.scale * r.scale) / 190e3;
+    if (us < kReadCutMin) return 0;
+    uint64_t total = 0, sum = 0;
+    for (const PassItem& p : items) total += (uint64_t)p.ctx->N;
+    for (uint32_t i = 0; i < (uint32_t)items.size(); i++) {
+        sum += (uint64_t)items[i].ctx->N;
+        if (sum * kReadCutDen >= total * kReadCutNum) return i + 1 < (uint32_t)items.size() ? i + 1 : 0;
+    }
+    return 0;
 }
 
 void release_contexts(fgc_batch* b) {
@@ -76,7 +139,7 @@ int issue(fgc_batch* b) {
     if (!b->use_graph) {
         rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, 0);
         if (rc) return rc;
-        rc = enqueue_reads(b);
+        rc = enqueue_all_reads(b);
         if (rc) return rc;
         FGC_CUDA(cudaEventRecord(b->done, b->stream));
         return FGC_OK;
@@ -86,7 +149,7 @@ int issue(fgc_batch* b) {
     // the new one has the same shape, otherwise instantiated anew.
     FGC_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, 0);
-    if (rc == FGC_OK) rc = enqueue_reads(b);
+    if (rc == FGC_OK) rc = enqueue_all_reads(b);
     cudaGraph_t g = nullptr;
     cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
     if (rc) {
@@ -134,7 +197,7 @@ int finish(fgc_batch* b) {
         // untouched; run them again with the sizes the device measured
         rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, from);
         if (rc) return rc;
-        rc = enqueue_reads(b);
+        rc = enqueue_all_reads(b);
         if (rc) return rc;
     }
     return fail(FGC_ERR_DEVICE_LIMIT, "draw buffers kept overflowing");
@@ -172,12 +235,18 @@ int submit(fgc_batch* b, const fgc_batch_item* items, uint64_t n) {
         if (it.out_nrgba) {
             const int32_t s = it.out_scale < 1 ? 1 : it.out_scale;
             if (c->W % s != 0 || c->H % s != 0) return fail(FGC_ERR_INVALID_ARGUMENT, "out_scale must divide the frame");
-            fgc_batch::ReadBack r{it.context, it.out_nrgba, s, ds_total};
+            fgc_batch::ReadBack r{it.context, (uint32_t)i, it.out_nrgba, s, ds_total};
             if (s > 1) ds_total += (size_t)(c->W / s) * (size_t)(c->H / s);
             b->reads.push_back(r);
         }
     }
     if (ds_total) FGC_CUDA(b->ds.ensure(ds_total));
+    sub.cut = read_cut(b);
+    if (sub.cut) {
+        if (!b->copy) FGC_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
+        if (!b->copied) FGC_CUDA(cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming));
+        if (!sub.at_cut) FGC_CUDA(cudaEventCreateWithFlags(&sub.at_cut, cudaEventDisableTiming));
+    }
     // claim the targets; the first draw on each takes its pending clears
     std::vector<fgc_context*> claimed;
     for (uint64_t i = 0; i < n; i++) {
@@ -269,6 +338,9 @@ int fgc_batch_destroy(fgc_batch* b) {
         cudaStreamSynchronize(b->stream);
         if (b->exec) cudaGraphExecDestroy(b->exec);
         if (b->done) cudaEventDestroy(b->done);
+        if (b->copied) cudaEventDestroy(b->copied);
+        if (b->sub.at_cut) cudaEventDestroy(b->sub.at_cut);
+        if (b->copy) cudaStreamDestroy(b->copy);
     }
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;

@@ -330,6 +330,8 @@ struct Submission {
     std::vector<PassRecord> passes;
     std::vector<fgc_rasterize_info> infos;
     std::vector<std::vector<cudaEvent_t>> events;  // stage boundaries per pass, when timing
+    uint32_t cut = 0;             // item that begins a pass of its own accord, or 0
+    cudaEvent_t at_cut = nullptr; // recorded before that pass
     fgc_stats stats = {};
     bool timing = false;
     Submission() = default;

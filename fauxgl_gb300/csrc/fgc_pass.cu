@@ -101,13 +101,13 @@ uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 // Draws go to the current pass until one repeats a target context (its
 // draws must run in order) or changes precision (one raster variant per
 // launch).
-std::vector<std::vector<uint32_t>> split_passes(const std::vector<PassItem>& items) {
+std::vector<std::vector<uint32_t>> split_passes(const std::vector<PassItem>& items, uint32_t cut) {
     std::vector<std::vector<uint32_t>> out;
     std::vector<const fgc_context*> seen;
     int prec = -1;
     for (uint32_t i = 0; i < (uint32_t)items.size(); i++) {
         const PassItem& it = items[i];
-        bool fresh = out.empty() || it.sv.precision != prec ||
+        bool fresh = out.empty() || it.sv.precision != prec || (cut && i == cut) ||
                      std::find(seen.begin(), seen.end(), it.ctx) != seen.end();
         if (fresh) {
             out.emplace_back();
@@ -335,7 +335,7 @@ namespace {
 int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, const Submission& sub,
                     std::vector<std::vector<uint32_t>>& groups, std::vector<PassPlan>& plans, uint32_t& nmax,
                     uint32_t& need_grid) {
-    groups = split_passes(sub.items);
+    groups = split_passes(sub.items, sub.cut);
     plans.assign(groups.size(), PassPlan{});
     nmax = 1;
     for (size_t g = 0; g < groups.size(); g++) {
@@ -456,6 +456,7 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
 
     for (size_t g = first_pass; g < plans.size(); g++) {
         const PassPlan& P = plans[g];
+        if (sub.cut && groups[g][0] == sub.cut) FGC_CUDA(cudaEventRecord(sub.at_cut, stream));
         PassRecord& rec = sub.passes[g];
         const uint32_t n = (uint32_t)P.views.size();
         rec.in_off = g * TL.in_bytes();
