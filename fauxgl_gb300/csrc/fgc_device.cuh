@@ -14,6 +14,7 @@
 #include "../../include/fauxglcuda.h"
 #include "fgc_certshade.cuh"
 #include "fgc_intconv.cuh"
+#include "fgc_softdiv.cuh"
 
 namespace fgc {
 
@@ -517,6 +518,8 @@ __device__ __forceinline__ D3 normalize3(D3 a) {
     double r = __drcp_rn(__dsqrt_rn(dot3(a, a)));  // 1 / sqrt(...), correctly rounded
     return muls3(a, r);
 }
+// The same where the FP64 pipe is the bound (fgc_softdiv.cuh).
+__device__ __forceinline__ D3 normalize3_busy(D3 a) { return muls3(a, rcp_i(sqrt_i(dot3(a, a)))); }
 
 __device__ __forceinline__ D4 d4(double x, double y, double z, double w) { return D4{x, y, z, w}; }
 __device__ __forceinline__ D4 add4(D4 a, D4 b) {
@@ -587,6 +590,9 @@ __device__ __forceinline__ double div_by_rcp(double x, double w, double y) {
 // with y = RN(1 / Output.W).
 __device__ __forceinline__ D3 ndc_of_rcp(D4 o, double y) {
     return d3(div_by_rcp(o.x, o.w, y), div_by_rcp(o.y, o.w, y), div_by_rcp(o.z, o.w, y));
+}
+__device__ __forceinline__ D3 ndc_of_soft(D4 o, const SoftRcp& r) {
+    return d3(div_of(o.x, o.w, r), div_of(o.y, o.w, r), div_of(o.z, o.w, r));
 }
 __device__ __forceinline__ D3 ndc_of(D4 o) { return ndc_of_rcp(o, __drcp_rn(o.w)); }
 

@@ -29,8 +29,9 @@ __global__ void __launch_bounds__(kVertexTile) vertex_kernel(VertexParams P) {
         const uint64_t o = I.vbase + u;
         P.vclip[o] = VClip{c.x, c.y, c.z, c.w};
         P.vout[o] = outside4(c) ? 1 : 0;
-        const double rw = __drcp_rn(c.w);
-        D3 n = ndc_of_rcp(c, rw);
+        const SoftRcp r = soft_rcp(c.w);
+        const double rw = rcp_of(c.w, r);
+        D3 n = ndc_of_soft(c, r);
         P.vndc[o] = make_double2(n.x, n.y);
         D3 s = screen_of_ndc(n, I.w2, I.h2);
         P.vscr[o] = VScreen{s.x, s.y, s.z, rw};
@@ -54,6 +55,19 @@ __device__ void write_dead(const GeomParams& P, uint64_t slot) {
     P.pbox[slot] = PBox{1, 0, 1, 0};
 }
 
+// BUSY: many primitives at once, so that the FP64 pipe bounds the kernel and
+// reciprocals are better formed on the integer pipe; a lone warp's FP64 chain
+// is the shorter one.
+template <bool BUSY>
+__device__ __forceinline__ double rcp_form(double x) {
+    return BUSY ? rcp_i(x) : __drcp_rn(x);  // 1 / x, correctly rounded
+}
+template <bool BUSY>
+__device__ __forceinline__ D3 normalize_form(D3 a) {
+    return BUSY ? normalize3_busy(a) : normalize3(a);
+}
+
+template <bool BUSY>
 __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s2, double r0, double r1,
                           double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem) {
     if (slot >= P.prim_cap) {  // slots reserved past an overflowing clip list
@@ -141,10 +155,10 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
             }
         }
     }
-    R.ra = __drcp_rn(area2);  // 1 / x, correctly rounded
-    R.q0 = __drcp_rn(a12);
-    R.q1 = __drcp_rn(a20);
-    R.q2 = __drcp_rn(a01);
+    R.ra = rcp_form<BUSY>(area2);
+    R.q0 = rcp_form<BUSY>(a12);
+    R.q1 = rcp_form<BUSY>(a20);
+    R.q2 = rcp_form<BUSY>(a01);
     R.z0 = s0.z; R.z1 = s1.z; R.z2 = s2.z;
     R.r0 = r0; R.r1 = r1; R.r2 = r2;
     R.v0 = v0; R.v1 = v1; R.v2 = v2;
@@ -174,6 +188,7 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
 
 // line (context.go:283-294): a screen-space quad of width LineWidth as two
 // raster primitives, (v1,v0,v0; s11,s01,s00) and (v1,v1,v0; s10,s11,s00).
+template <bool BUSY>
 __device__ void make_line_prims(const GeomParams& P, double line_width, uint64_t slot, D3 s0, D3 s1, double r0,
                                 double r1, uint32_t v0, uint32_t v1, uint32_t elem) {
     double lw2 = __ddiv_rn(line_width, 2.0);
@@ -182,17 +197,17 @@ __device__ void make_line_prims(const GeomParams& P, double line_width, uint64_t
     if (d.x == 0 && d.y == 0) {
         perp = (d.z == 0) ? d3(0, 0, 0) : d3(0, 1, 0);
     } else {
-        perp = normalize3(d3(-d.y, d.x, 0.0));
+        perp = normalize_form<BUSY>(d3(-d.y, d.x, 0.0));
     }
     D3 n = muls3(perp, lw2);
-    s0 = add3(s0, muls3(normalize3(sub3(s0, s1)), lw2));
-    s1 = add3(s1, muls3(normalize3(sub3(s1, s0)), lw2));
+    s0 = add3(s0, muls3(normalize_form<BUSY>(sub3(s0, s1)), lw2));
+    s1 = add3(s1, muls3(normalize_form<BUSY>(sub3(s1, s0)), lw2));
     D3 s00 = add3(s0, n);
     D3 s01 = sub3(s0, n);
     D3 s10 = add3(s1, n);
     D3 s11 = sub3(s1, n);
-    make_prim(P, slot, s11, s01, s00, r1, r0, r0, v1, v0, v0, elem);
-    make_prim(P, slot + 1, s10, s11, s00, r1, r1, r0, v1, v1, v0, elem);
+    make_prim<BUSY>(P, slot, s11, s01, s00, r1, r0, r0, v1, v0, v0, elem);
+    make_prim<BUSY>(P, slot + 1, s10, s11, s00, r1, r1, r0, v1, v1, v0, elem);
 }
 
 // clipPlanes (clipping.go:3-10): {P, N} of +x, -x, +y, -y, +z, -z.
@@ -264,11 +279,11 @@ __device__ __forceinline__ int cull_decision(const StateView& st, double n0x, do
 __device__ void emit_triangle(const GeomParams& P, const StateView& st, uint64_t slot, D3 s0, D3 s1, D3 s2,
                               double r0, double r1, double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem) {
     if (st.wireframe) {
-        make_line_prims(P, st.line_width, slot + 0, s0, s1, r0, r1, v0, v1, elem);
-        make_line_prims(P, st.line_width, slot + 2, s1, s2, r1, r2, v1, v2, elem);
-        make_line_prims(P, st.line_width, slot + 4, s2, s0, r2, r0, v2, v0, elem);
+        make_line_prims<false>(P, st.line_width, slot + 0, s0, s1, r0, r1, v0, v1, elem);
+        make_line_prims<false>(P, st.line_width, slot + 2, s1, s2, r1, r2, v1, v2, elem);
+        make_line_prims<false>(P, st.line_width, slot + 4, s2, s0, r2, r0, v2, v0, elem);
     } else {
-        make_prim(P, slot, s0, s1, s2, r0, r1, r2, v0, v1, v2, elem);
+        make_prim<false>(P, slot, s0, s1, s2, r0, r1, r2, v0, v1, v2, elem);
     }
 }
 
@@ -297,7 +312,7 @@ __device__ void emit_triangle_piece(const GeomParams& P, const ItemView& I, uint
     const VScreen* vscr = P.vscr + I.vbase;
     if (!I.st.wireframe) {
         const VScreen a = vscr[u0], b = vscr[u1], c = vscr[u2];
-        make_prim(P, slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), d3(c.x, c.y, c.z), a.rw, b.rw, c.rw, c0, c1, c2,
+        make_prim<true>(P, slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), d3(c.x, c.y, c.z), a.rw, b.rw, c.rw, c0, c1, c2,
                   (uint32_t)t);
         return;
     }
@@ -307,7 +322,7 @@ __device__ void emit_triangle_piece(const GeomParams& P, const ItemView& I, uint
     const uint32_t ca = piece == 0 ? c0 : piece == 1 ? c1 : c2;
     const uint32_t cb = piece == 0 ? c1 : piece == 1 ? c2 : c0;
     const VScreen a = vscr[ua], b = vscr[ub];
-    make_line_prims(P, I.st.line_width, slot + 2 * piece, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw, ca, cb,
+    make_line_prims<true>(P, I.st.line_width, slot + 2 * piece, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw, ca, cb,
                     (uint32_t)t);
 }
 
@@ -527,7 +542,7 @@ __global__ void __launch_bounds__(256, 3) setup_emit_kernel(GeomParams P) {
             const uint64_t cb = 3 * I.mesh.ntri + 2 * (uint64_t)w.elem;
             const VScreen* vscr = P.vscr + I.vbase;
             const VScreen a = vscr[w.u0], b = vscr[w.u1];
-            make_line_prims(P, I.st.line_width, w.slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw,
+            make_line_prims<true>(P, I.st.line_width, w.slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw,
                             (uint32_t)cb, (uint32_t)(cb + 1), kLineFlag | w.elem);
         } else {
             const int order = (int)((w.meta >> 8) & 0xFFu) - 1;
@@ -899,7 +914,7 @@ __global__ void __launch_bounds__(128) clip_lines_kernel(GeomParams P) {
         }
         D3 s0 = screen_of_ndc(ndc_of(w1), I.w2, I.h2);
         D3 s1 = screen_of_ndc(ndc_of(w2), I.w2, I.h2);
-        make_line_prims(P, I.st.line_width, slot, s0, s1, __ddiv_rn(1.0, w1.w), __ddiv_rn(1.0, w2.w), (uint32_t)cb,
+        make_line_prims<false>(P, I.st.line_width, slot, s0, s1, __ddiv_rn(1.0, w1.w), __ddiv_rn(1.0, w2.w), (uint32_t)cb,
                         (uint32_t)(cb + 1), kLineFlag | (uint32_t)l);
     }
 }

@@ -165,7 +165,7 @@ __device__ __noinline__ D4 shade64(const RasterParams& P, const ItemView& I, con
     if (S.kind == FGC_SHADER_SOLID_COLOR) return d4(S.color[0], S.color[1], S.color[2], S.color[3]);
     // perspective-correct barycentrics (context.go:236-237)
     D4 w = d4(__dmul_rn(b0, R.r0), __dmul_rn(b1, R.r1), __dmul_rn(b2, R.r2), 0.0);
-    w.w = __drcp_rn(__dadd_rn(__dadd_rn(w.x, w.y), w.z));
+    w.w = rcp_i(__dadd_rn(__dadd_rn(w.x, w.y), w.z));
     if (S.kind == FGC_SHADER_TEXTURE) {
         double u0, v0, u1, v1, u2, v2;
         fetch_tex64(P, M, R.v0, u0, v0);
@@ -178,7 +178,7 @@ __device__ __noinline__ D4 shade64(const RasterParams& P, const ItemView& I, con
     fetch_pn64(P, M, R.v0, p0, n0);
     fetch_pn64(P, M, R.v1, p1, n1);
     fetch_pn64(P, M, R.v2, p2, n2);
-    D3 nrm = normalize3(d3(interp1(n0.x, n1.x, n2.x, w), interp1(n0.y, n1.y, n2.y, w), interp1(n0.z, n1.z, n2.z, w)));
+    D3 nrm = normalize3_busy(d3(interp1(n0.x, n1.x, n2.x, w), interp1(n0.y, n1.y, n2.y, w), interp1(n0.z, n1.z, n2.z, w)));
     D4 color;
     if (S.object_is_discard) {
         D4 c0 = fetch_col64(P, M, R.v0), c1 = fetch_col64(P, M, R.v1), c2 = fetch_col64(P, M, R.v2);
@@ -210,7 +210,7 @@ __device__ __noinline__ D4 shade64(const RasterParams& P, const ItemView& I, con
     if (dgt0(diffuse) && S.power_pos) {
         // the interpolated position is read only here
         const D3 pos = d3(interp1(p0.x, p1.x, p2.x, w), interp1(p0.y, p1.y, p2.y, w), interp1(p0.z, p1.z, p2.z, w));
-        D3 camera = normalize3(sub3(d3(S.eye[0], S.eye[1], S.eye[2]), pos));
+        D3 camera = normalize3_busy(sub3(d3(S.eye[0], S.eye[1], S.eye[2]), pos));
         D3 negl = d3(-L.x, -L.y, -L.z);
         // Reflect (vector.go:175-177) with n.Dot(-L) = -(n.Dot(L)): rounding is
         // symmetric, so the two differ at most in the sign of a zero, which
