@@ -67,17 +67,20 @@ __device__ __forceinline__ D3 normalize_form(D3 a) {
     return BUSY ? normalize3_busy(a) : normalize3(a);
 }
 
+// Forms the primitive's record in R and writes the rest of its slot. False
+// when the slot is dead or does not exist.
 template <bool BUSY>
-__device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s2, double r0, double r1,
-                          double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem) {
+__device__ __forceinline__ bool build_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s2, double r0,
+                                           double r1, double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem,
+                                           RPrim& R) {
     if (slot >= P.prim_cap) {  // slots reserved past an overflowing clip list
         atomicOr(P.status, ST_CLIP_OVERFLOW);
-        return;
+        return false;
     }
     if (!(dfinite(s0.x) && dfinite(s0.y) && dfinite(s0.z) && dfinite(s1.x) && dfinite(s1.y) && dfinite(s1.z) &&
           dfinite(s2.x) && dfinite(s2.y) && dfinite(s2.z))) {
         write_dead(P, slot);
-        return;
+        return false;
     }
     // integer bounding box (Min/Max, Floor/Ceil, int())
     const int64_t x0 = go_floor_i(go_min_i(s0.x, go_min_i(s1.x, s2.x)));
@@ -87,26 +90,23 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
     const int64_t lim = 1LL << 30;
     if (x1 - x0 > kMaxExtent || y1 - y0 > kMaxExtent || x0 < -lim || x1 > lim || y0 < -lim || y1 > lim) {
         write_dead(P, slot);
-        return;
+        return false;
     }
     D3 p = d3(__dadd_rn(i2d_i(x0), 0.5), __dadd_rn(i2d_i(y0), 0.5), 0.0);  // |x0|, |y0| <= 2^30 here
-    RPrim R;
     // edge(a, b, p) = (b.X - p.X)(a.Y - p.Y) - (b.Y - p.Y)(a.X - p.X)
     // (context.go:147-149): the six differences to p are shared by the three
     // edges
     const double dx0 = __dsub_rn(s0.x, p.x), dx1 = __dsub_rn(s1.x, p.x), dx2 = __dsub_rn(s2.x, p.x);
     const double dy0 = __dsub_rn(s0.y, p.y), dy1 = __dsub_rn(s1.y, p.y), dy2 = __dsub_rn(s2.y, p.y);
-    R.w0 = __dsub_rn(__dmul_rn(dx2, dy1), __dmul_rn(dy2, dx1));  // edge(s1, s2, p)
-    R.w1 = __dsub_rn(__dmul_rn(dx0, dy2), __dmul_rn(dy0, dx2));  // edge(s2, s0, p)
-    R.w2 = __dsub_rn(__dmul_rn(dx1, dy0), __dmul_rn(dy1, dx0));  // edge(s0, s1, p)
+    double w0 = __dsub_rn(__dmul_rn(dx2, dy1), __dmul_rn(dy2, dx1));  // edge(s1, s2, p)
+    double w1 = __dsub_rn(__dmul_rn(dx0, dy2), __dmul_rn(dy0, dx2));  // edge(s2, s0, p)
+    double w2 = __dsub_rn(__dmul_rn(dx1, dy0), __dmul_rn(dy1, dx0));  // edge(s0, s1, p)
     double a01 = __dsub_rn(s1.y, s0.y);
     double b01 = __dsub_rn(s0.x, s1.x);
     double a12 = __dsub_rn(s2.y, s1.y);
     double b12 = __dsub_rn(s1.x, s2.x);
     double a20 = __dsub_rn(s0.y, s2.y);
     double b20 = __dsub_rn(s2.x, s0.x);
-    R.a0 = a12; R.a1 = a20; R.a2 = a01;
-    R.b0 = b12; R.b1 = b20; R.b2 = b01;
     // edge(s0, s1, s2) = (s1.X - s2.X)(s0.Y - s2.Y) - (s1.Y - s2.Y)(s0.X - s2.X):
     // its factors are b12, a20, -a12 and -b20 (a rounded difference changes
     // only its sign when the operands swap), and (-a12)(-b20) = a12 b20
@@ -146,15 +146,18 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
             rx1 = x1 - 1 - (dgt_i(__dsub_rn(i2d_i(x1), xmax), kHalfEps) ? 1 : 0);
             if (ry0 > ry1 || rx1 < x0) {
                 write_dead(P, slot);  // no pixel centre can be covered
-                return;
+                return false;
             }
             if (ry0 > y0) {  // w00 += b12 etc. (context.go:275-277) for the row left out
-                R.w0 = __dadd_rn(R.w0, b12);
-                R.w1 = __dadd_rn(R.w1, b20);
-                R.w2 = __dadd_rn(R.w2, b01);
+                w0 = __dadd_rn(w0, b12);
+                w1 = __dadd_rn(w1, b20);
+                w2 = __dadd_rn(w2, b01);
             }
         }
     }
+    R.w0 = w0; R.w1 = w1; R.w2 = w2;
+    R.a0 = a12; R.a1 = a20; R.a2 = a01;
+    R.b0 = b12; R.b1 = b20; R.b2 = b01;
     R.ra = rcp_form<BUSY>(area2);
     R.q0 = rcp_form<BUSY>(a12);
     R.q1 = rcp_form<BUSY>(a20);
@@ -163,7 +166,6 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
     R.r0 = r0; R.r1 = r1; R.r2 = r2;
     R.v0 = v0; R.v1 = v1; R.v2 = v2;
     R.elem = elem;
-    P.prims[slot] = R;
     P.pbox[slot] = PBox{(int32_t)x0, (int32_t)rx1, (int32_t)ry0, (int32_t)ry1};
     P.rf[slot] = make_float4((float)r0, (float)r1, (float)r2, 0.0f);
     // A row's covered pixel centres lie on one horizontal chord of the
@@ -184,13 +186,23 @@ __device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s
         if (s < (float)bw) span = (uint32_t)s;
     }
     P.pspan[slot] = span;
+    return true;
+}
+
+template <bool BUSY>
+__device__ void make_prim(const GeomParams& P, uint64_t slot, D3 s0, D3 s1, D3 s2, double r0, double r1,
+                          double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem) {
+    RPrim R;
+    if (build_prim<BUSY>(P, slot, s0, s1, s2, r0, r1, r2, v0, v1, v2, elem, R)) P.prims[slot] = R;
 }
 
 // line (context.go:283-294): a screen-space quad of width LineWidth as two
 // raster primitives, (v1,v0,v0; s11,s01,s00) and (v1,v1,v0; s10,s11,s00).
+struct LineCorners {
+    D3 s00, s01, s10, s11;
+};
 template <bool BUSY>
-__device__ void make_line_prims(const GeomParams& P, double line_width, uint64_t slot, D3 s0, D3 s1, double r0,
-                                double r1, uint32_t v0, uint32_t v1, uint32_t elem) {
+__device__ __forceinline__ LineCorners line_corners(double line_width, D3 s0, D3 s1) {
     double lw2 = __ddiv_rn(line_width, 2.0);
     D3 d = sub3(s1, s0);
     D3 perp;  // Perpendicular (vector.go:179-187)
@@ -202,12 +214,13 @@ __device__ void make_line_prims(const GeomParams& P, double line_width, uint64_t
     D3 n = muls3(perp, lw2);
     s0 = add3(s0, muls3(normalize_form<BUSY>(sub3(s0, s1)), lw2));
     s1 = add3(s1, muls3(normalize_form<BUSY>(sub3(s1, s0)), lw2));
-    D3 s00 = add3(s0, n);
-    D3 s01 = sub3(s0, n);
-    D3 s10 = add3(s1, n);
-    D3 s11 = sub3(s1, n);
-    make_prim<BUSY>(P, slot, s11, s01, s00, r1, r0, r0, v1, v0, v0, elem);
-    make_prim<BUSY>(P, slot + 1, s10, s11, s00, r1, r1, r0, v1, v1, v0, elem);
+    return LineCorners{add3(s0, n), sub3(s0, n), add3(s1, n), sub3(s1, n)};
+}
+__device__ void make_line_prims(const GeomParams& P, double line_width, uint64_t slot, D3 s0, D3 s1, double r0,
+                                double r1, uint32_t v0, uint32_t v1, uint32_t elem) {
+    const LineCorners c = line_corners<false>(line_width, s0, s1);
+    make_prim<false>(P, slot, c.s11, c.s01, c.s00, r1, r0, r0, v1, v0, v0, elem);
+    make_prim<false>(P, slot + 1, c.s10, c.s11, c.s00, r1, r1, r0, v1, v1, v0, elem);
 }
 
 // clipPlanes (clipping.go:3-10): {P, N} of +x, -x, +y, -y, +z, -z.
@@ -279,9 +292,9 @@ __device__ __forceinline__ int cull_decision(const StateView& st, double n0x, do
 __device__ void emit_triangle(const GeomParams& P, const StateView& st, uint64_t slot, D3 s0, D3 s1, D3 s2,
                               double r0, double r1, double r2, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t elem) {
     if (st.wireframe) {
-        make_line_prims<false>(P, st.line_width, slot + 0, s0, s1, r0, r1, v0, v1, elem);
-        make_line_prims<false>(P, st.line_width, slot + 2, s1, s2, r1, r2, v1, v2, elem);
-        make_line_prims<false>(P, st.line_width, slot + 4, s2, s0, r2, r0, v2, v0, elem);
+        make_line_prims(P, st.line_width, slot + 0, s0, s1, r0, r1, v0, v1, elem);
+        make_line_prims(P, st.line_width, slot + 2, s1, s2, r1, r2, v1, v2, elem);
+        make_line_prims(P, st.line_width, slot + 4, s2, s0, r2, r0, v2, v0, elem);
     } else {
         make_prim<false>(P, slot, s0, s1, s2, r0, r1, r2, v0, v1, v2, elem);
     }
@@ -299,32 +312,6 @@ __device__ void emit_triangle(const GeomParams& P, const StateView& st, uint64_t
 // setup_emit_kernel turns into raster primitives, while the clip kernels (on
 // another stream) handle the clip entries.
 // ---------------------------------------------------------------------------
-
-// One piece of a triangle that survived culling: the whole triangle, or in
-// wireframe its edge `piece` (two primitives at slot + 2*piece).
-__device__ void emit_triangle_piece(const GeomParams& P, const ItemView& I, uint64_t t, uint64_t slot, int order,
-                                    uint32_t u0, uint32_t u1, uint32_t u2, uint32_t piece) {
-    uint32_t c0 = (uint32_t)(3 * t), c1 = c0 + 1, c2 = c0 + 2;
-    if (order < 0) {  // swap v0 <-> v2
-        uint32_t tu = u0; u0 = u2; u2 = tu;
-        uint32_t tc = c0; c0 = c2; c2 = tc;
-    }
-    const VScreen* vscr = P.vscr + I.vbase;
-    if (!I.st.wireframe) {
-        const VScreen a = vscr[u0], b = vscr[u1], c = vscr[u2];
-        make_prim<true>(P, slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), d3(c.x, c.y, c.z), a.rw, b.rw, c.rw, c0, c1, c2,
-                  (uint32_t)t);
-        return;
-    }
-    // wireframe: line(v0, v1), line(v1, v2), line(v2, v0) (context.go:296-301)
-    const uint32_t ua = piece == 0 ? u0 : piece == 1 ? u1 : u2;
-    const uint32_t ub = piece == 0 ? u1 : piece == 1 ? u2 : u0;
-    const uint32_t ca = piece == 0 ? c0 : piece == 1 ? c1 : c2;
-    const uint32_t cb = piece == 0 ? c1 : piece == 1 ? c2 : c0;
-    const VScreen a = vscr[ua], b = vscr[ub];
-    make_line_prims<true>(P, I.st.line_width, slot + 2 * piece, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw, ca, cb,
-                    (uint32_t)t);
-}
 
 // One element's setup decision: its primitive slots (count), the
 // primitive-emitting pieces it hands to the emit kernel (work: a triangle,
@@ -526,7 +513,37 @@ __global__ void __launch_bounds__(kSetupTile) setup_kernel(GeomParams P) {
 
 // The FP64 half of setup: one thread per work item, every lane busy (the
 // work list holds only what survived culling), no barriers.
+__device__ __forceinline__ VScreen load_screen(const VScreen* p) {  // 32 bytes by one load
+    VScreen v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.rw) : "l"(p));
+    return v;
+}
+
+constexpr int kRecVec = sizeof(RPrim) / 16;  // 16-byte parts of a record
+
+// Writes the records that a warp's lanes formed in shared memory (ok: the lane
+// has one, for its slot), in the order of the slots, which mostly follow each
+// other. Written lane by lane each of the eleven stores of a record touched 32
+// lines, and memory stalls were half of the kernel's: setup of 1.3 M triangles
+// 145 -> 130 us, of a 16x supersampled wireframe (2.5 M primitives) 495 -> 453.
+// The FP64 pipe is busy for half of the rest. (A record in registers first: 143
+// and 476 us at two blocks per SM, spills at three; the next item's vertices
+// loaded ahead in a resident grid: 150 and 515.)
+__device__ __forceinline__ void store_records(const GeomParams& P, const uint4* s_rec, bool ok, uint32_t slot) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t m = __ballot_sync(0xffffffffu, ok);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kRecVec; j++) {
+        const uint32_t c = (uint32_t)j * 32 + lane, rec = c / kRecVec, part = c % kRecVec;
+        const uint32_t to = __shfl_sync(0xffffffffu, slot, (int)rec);
+        if ((m >> rec) & 1u) reinterpret_cast<uint4*>(&P.prims[to])[part] = s_rec[c];
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(256, 3) setup_emit_kernel(GeomParams P) {
+    __shared__ __align__(16) RPrim s_rec[256];
     // a look-back wait that gave up (a scan of an earlier pass) leaves the
     // pass to be reported as failed: emit nothing
     if (*P.status & ST_LOOKBACK_TIMEOUT) return;
@@ -534,19 +551,84 @@ __global__ void __launch_bounds__(256, 3) setup_emit_kernel(GeomParams P) {
         for (uint32_t i = threadIdx.x; i < P.nitems; i += blockDim.x)
             P.iout[i].prim_end = (i + 1 < P.nitems) ? P.iout[i + 1].prim_start : *P.prim_total;
     const uint64_t n = min((uint64_t)*P.work_total, P.work_cap);
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const SetupWork w = P.work[i];
-        const ItemView& I = P.items[w.item];
-        const uint32_t piece = w.meta & 0xFFu;
-        if (w.meta & kWorkLine) {
-            const uint64_t cb = 3 * I.mesh.ntri + 2 * (uint64_t)w.elem;
+    const uint32_t lane = threadIdx.x & 31;
+    // a warp's lanes stay together: they write their records jointly
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
+         i0 += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t prims = 0, slot = 0, elem = 0;
+        // corners and vertices of the item's first primitive, for a line also
+        // the fourth corner (s10) of its second
+        D3 s0 = d3(0, 0, 0), s1 = s0, s2 = s0, s3 = s0;
+        double r0 = 0, r1 = 0, r2 = 0;
+        uint32_t v0 = 0, v1 = 0, v2 = 0;
+        if (i0 + lane < n) {
+            const SetupWork w = P.work[i0 + lane];
+            const ItemView& I = P.items[w.item];
             const VScreen* vscr = P.vscr + I.vbase;
-            const VScreen a = vscr[w.u0], b = vscr[w.u1];
-            make_line_prims<true>(P, I.st.line_width, w.slot, d3(a.x, a.y, a.z), d3(b.x, b.y, b.z), a.rw, b.rw,
-                            (uint32_t)cb, (uint32_t)(cb + 1), kLineFlag | w.elem);
-        } else {
-            const int order = (int)((w.meta >> 8) & 0xFFu) - 1;
-            emit_triangle_piece(P, I, w.elem, w.slot, order, w.u0, w.u1, w.u2, piece);
+            const bool is_line = (w.meta & kWorkLine) != 0;
+            slot = (uint32_t)w.slot;  // below 2^31, as every slot
+            elem = w.elem;
+            // the whole triangle, an edge of a wireframe triangle, or a line
+            uint32_t ua = w.u0, ub = w.u1, ca, cb;
+            if (is_line) {
+                ca = (uint32_t)(3 * I.mesh.ntri + 2 * (uint64_t)w.elem);
+                cb = ca + 1;
+                elem |= kLineFlag;
+            } else {
+                uint32_t u0 = w.u0, u1 = w.u1, u2 = w.u2, c0 = (uint32_t)(3 * (uint64_t)w.elem), c1 = c0 + 1, c2 = c0 + 2;
+                if (((w.meta >> 8) & 0xFFu) == 0u) {  // order -1: swap v0 <-> v2
+                    uint32_t tu = u0; u0 = u2; u2 = tu;
+                    uint32_t tc = c0; c0 = c2; c2 = tc;
+                }
+                // wireframe: line(v0, v1), line(v1, v2), line(v2, v0) (context.go:296-301)
+                const uint32_t piece = w.meta & 0xFFu;
+                ua = piece == 0 ? u0 : piece == 1 ? u1 : u2;
+                ub = piece == 0 ? u1 : piece == 1 ? u2 : u0;
+                ca = piece == 0 ? c0 : piece == 1 ? c1 : c2;
+                cb = piece == 0 ? c1 : piece == 1 ? c2 : c0;
+                if (I.st.wireframe) {
+                    slot += 2 * piece;
+                } else {
+                    const VScreen c = load_screen(vscr + u2);
+                    s2 = d3(c.x, c.y, c.z);
+                    r2 = c.rw;
+                    v2 = c2;
+                    prims = 1;
+                }
+            }
+            const VScreen a = load_screen(vscr + ua), b = load_screen(vscr + ub);
+            s0 = d3(a.x, a.y, a.z);
+            s1 = d3(b.x, b.y, b.z);
+            r0 = a.rw;
+            r1 = b.rw;
+            v0 = ca;
+            v1 = cb;
+            if (prims == 0) {  // (v1, v0, v0; s11, s01, s00)
+                prims = 2;
+                const LineCorners c = line_corners<true>(I.st.line_width, s0, s1);
+                s0 = c.s11;
+                s1 = c.s01;
+                s2 = c.s00;
+                s3 = c.s10;
+                r2 = r0;
+                r0 = r1;
+                r1 = r2;
+                v2 = v0;
+                v0 = v1;
+                v1 = v2;
+            }
+        }
+#pragma unroll 1
+        for (uint32_t p = 0; __any_sync(0xffffffffu, p < prims); p++) {
+            const bool ok = p < prims && build_prim<true>(P, slot, s0, s1, s2, r0, r1, r2, v0, v1, v2, elem,
+                                                          s_rec[threadIdx.x]);
+            store_records(P, reinterpret_cast<const uint4*>(&s_rec[threadIdx.x & ~31u]), ok, slot);
+            // the line's second primitive: (v1, v1, v0; s10, s11, s00)
+            slot++;
+            s1 = s0;
+            s0 = s3;
+            r1 = r0;
+            v1 = v0;
         }
     }
 }
@@ -914,7 +996,7 @@ __global__ void __launch_bounds__(128) clip_lines_kernel(GeomParams P) {
         }
         D3 s0 = screen_of_ndc(ndc_of(w1), I.w2, I.h2);
         D3 s1 = screen_of_ndc(ndc_of(w2), I.w2, I.h2);
-        make_line_prims<false>(P, I.st.line_width, slot, s0, s1, __ddiv_rn(1.0, w1.w), __ddiv_rn(1.0, w2.w), (uint32_t)cb,
+        make_line_prims(P, I.st.line_width, slot, s0, s1, __ddiv_rn(1.0, w1.w), __ddiv_rn(1.0, w2.w), (uint32_t)cb,
                         (uint32_t)(cb + 1), kLineFlag | (uint32_t)l);
     }
 }
