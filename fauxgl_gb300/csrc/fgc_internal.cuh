@@ -212,7 +212,7 @@ struct RowStartParams {
     const uint32_t* prs;        // exclusive scan of pnb
     const unsigned long long* prim_total;
     uint64_t cap;               // row-start slots (the bin capacity)
-    double* rstart;             // [slot][3]
+    double* rstart;             // [slot][4], the last unused
     unsigned int* status;
 };
 

@@ -382,7 +382,7 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
     FGC_CUDA(S.bins.ensure(S.bin_cap));
     FGC_CUDA(S.pnb.ensure(need_prims));
     FGC_CUDA(S.prs.ensure(need_prims));
-    FGC_CUDA(S.rstart.ensure(3 * S.bin_cap));
+    FGC_CUDA(S.rstart.ensure(4 * S.bin_cap));
     FGC_CUDA(S.tiles.ensure(need_tiles));
     FGC_CUDA(S.work.ensure(need_work));
     uint64_t need_stiles = 1;

@@ -434,7 +434,7 @@ __device__ __forceinline__ int64_t row_from(const RasterParams& P, uint32_t pp, 
         const BandGeom G{I.W, I.H, I.R, I.nbands};
         uint32_t bl = 0, bh = 0;
         prim_bands(G, bx, bl, bh);  // the primitive is binned to this band: bl <= B.band
-        rs = P.rstart + 3 * ((uint64_t)P.prs[pp] + (B.band - bl));
+        rs = P.rstart + 4 * ((uint64_t)P.prs[pp] + (B.band - bl));
         first = (int64_t)B.r0 - floordiv_w(bx.x1, I.W);
         if (first < bx.y0) first = bx.y0;
     }
@@ -446,9 +446,14 @@ __device__ __forceinline__ void row_start(const RasterParams& P, uint32_t pp, co
                                           double& w02) {
     const double* rs;
     const int64_t r = row_from(P, pp, bx, y, I, B, rs);
-    w00 = rs ? rs[0] : R.w0;
-    w01 = rs ? rs[1] : R.w1;
-    w02 = rs ? rs[2] : R.w2;
+    if (rs) {
+        double unused;
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(w00), "=d"(w01), "=d"(w02), "=d"(unused) : "l"(rs));
+    } else {
+        w00 = R.w0;
+        w01 = R.w1;
+        w02 = R.w2;
+    }
     if (r > 64) {
         w00 = repeat_add(w00, R.b0, (uint64_t)r);
         w01 = repeat_add(w01, R.b1, (uint64_t)r);
