@@ -562,9 +562,12 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
             // over every SM's FP64 pipes, and kClipSmall of them have a warp
             // each
             clip_poly_kernel<<<D.sms * 16, 32, 0, S.side>>>(gp);
-            clip_vert_kernel<<<grid_for((uint64_t)S.clip_cap * kClipPoly, 64, D.sms * 8), 64, 0, S.side>>>(gp);
+            rec.launches++;
+            if (S.clip_cap > kClipSmall) {  // else the list holds no more than clip_poly_kernel finishes
+                clip_vert_kernel<<<grid_for((uint64_t)S.clip_cap * kClipPoly, 64, D.sms * 8), 64, 0, S.side>>>(gp);
+                rec.launches++;
+            }
             FGC_CUDA(cudaGetLastError());
-            rec.launches += 2;
         }
         setup_scan_kernel<<<1, 1024, 0, stream>>>(gp);
         setup_kernel<<<P.stiles, kSetupTile, 0, stream>>>(gp);
