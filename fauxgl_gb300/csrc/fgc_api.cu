@@ -94,6 +94,21 @@ cudaError_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s) {
 
 void pool_free(void* p, cudaStream_t s) { cudaFreeAsync(p, s); }
 
+cudaError_t big_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    DevicePool* P = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        e = device_pool(&P);
+    }
+    if (e != cudaSuccess) return e;
+    cudaDeviceSynchronize();
+    for (cudaMemPool_t pool : P->pool) cudaMemPoolTrimTo(pool, 0);
+    return cudaMalloc(p, bytes);
+}
+
 cudaError_t take_stream(int device, cudaStream_t* s) {
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
