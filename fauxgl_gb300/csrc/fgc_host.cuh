@@ -300,7 +300,6 @@ struct PassScratch {
     DevBuf<uint32_t> mat, off, bins;
     DevBuf<uint32_t> pnb, prs;     // per primitive: bands it is binned to, first row-start slot
     DevBuf<double> rstart;         // per (primitive, band): edge values at its first row in the band
-    DevBuf<unsigned long long> tiles;
     DevBuf<unsigned char> table;   // item views + lookup starts + per-draw results + counters + status
     DevBuf<double> dbg;
     DevBuf<PendFrag> pend;         // per raster CTA: fragments awaiting their FP64 colour

@@ -46,19 +46,22 @@ static_assert(sizeof(PassHeader) == kHeaderBytes, "pass header layout");
 size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Device table of a submission (sized for its largest pass):
-//   [header][ItemOut x nmax][ItemView x nmax][4 lookup arrays of nmax + 1]
+//   [header][ItemOut x nmax][look-back tiles][ItemView x nmax][4 lookup arrays of nmax + 1]
 struct TableLayout {
     uint32_t nmax = 0;
-    size_t iout = 0, views = 0, starts = 0, total = 0;
-    size_t in_bytes() const { return total - views; }        // uploaded per pass
+    size_t iout = 0, tiles = 0, views = 0, starts = 0, total = 0;
     size_t out_bytes(uint32_t n) const { return iout + (size_t)n * sizeof(ItemOut); }
 };
 
-TableLayout table_layout(uint32_t nmax) {
+// Zeros before the uploaded tables that are uploaded with them at most.
+constexpr size_t kUploadZeros = 32 * 1024;
+
+TableLayout table_layout(uint32_t nmax, uint64_t ntiles) {
     TableLayout t;
     t.nmax = nmax;
     t.iout = kHeaderBytes;
-    t.views = align16(t.iout + (size_t)nmax * sizeof(ItemOut));
+    t.tiles = align16(t.iout + (size_t)nmax * sizeof(ItemOut));
+    t.views = align16(t.tiles + ntiles * sizeof(unsigned long long));
     t.starts = t.views + (size_t)nmax * sizeof(ItemView);
     t.total = align16(t.starts + 4 * sizeof(uint32_t) * ((size_t)nmax + 1));
     return t;
@@ -334,7 +337,7 @@ namespace {
 // issued (passes issued earlier on the stream may still be using them).
 int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, const Submission& sub,
                     std::vector<std::vector<uint32_t>>& groups, std::vector<PassPlan>& plans, uint32_t& nmax,
-                    uint32_t& need_grid) {
+                    uint32_t& need_grid, TableLayout& TL) {
     groups = split_passes(sub.items, sub.cut);
     plans.assign(groups.size(), PassPlan{});
     nmax = 1;
@@ -343,7 +346,6 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
         if (rc) return rc;
         nmax = std::max<uint32_t>(nmax, (uint32_t)groups[g].size());
     }
-    const TableLayout TL = table_layout(nmax);
     uint64_t need_prims = 0, need_vert = 1, need_lines = 1, need_mat = 1, need_tiles = 4, need_work = 1;
     bool need_dbg = false;
     need_grid = 1;
@@ -358,6 +360,7 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
         need_grid = std::max<uint32_t>(need_grid, std::min<uint32_t>(2 * D.sms, P.nbands));
         need_work = std::max<uint64_t>(need_work, P.work_items);
     }
+    TL = table_layout(nmax, need_tiles);
     // setup's ordered allocation carries the slot and work prefixes in 31
     // bits each
     if (need_prims >= (1ull << 31) || need_work >= (1ull << 31))
@@ -383,7 +386,6 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
     FGC_CUDA(S.pnb.ensure(need_prims));
     FGC_CUDA(S.prs.ensure(need_prims));
     FGC_CUDA(S.rstart.ensure(4 * S.bin_cap));
-    FGC_CUDA(S.tiles.ensure(need_tiles));
     FGC_CUDA(S.work.ensure(need_work));
     uint64_t need_stiles = 1;
     for (const PassPlan& P : plans) need_stiles = std::max<uint64_t>(need_stiles, P.stiles);
@@ -410,7 +412,7 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
         FGC_CUDA(cudaEventCreateWithFlags(&S.ev_join, cudaEventDisableTiming));
         S.side_device = dev;
     }
-    FGC_CUDA(S.host_in.ensure(TL.in_bytes() * plans.size()));
+    FGC_CUDA(S.host_in.ensure(TL.total * plans.size()));
     FGC_CUDA(S.host_out.ensure(TL.out_bytes(nmax) * plans.size()));
     size_t need_pend = 0;
     for (const PassPlan& P : plans)
@@ -430,7 +432,8 @@ int prepare_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, 
     std::vector<std::vector<uint32_t>> groups;
     std::vector<PassPlan> plans;
     uint32_t nmax = 1, need_grid = 1;
-    return plan_submission(S, D, T, sub, groups, plans, nmax, need_grid);
+    TableLayout TL;
+    return plan_submission(S, D, T, sub, groups, plans, nmax, need_grid, TL);
 }
 
 int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, const PassTuning& T, Submission& sub,
@@ -439,7 +442,8 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
     std::vector<std::vector<uint32_t>> groups;
     std::vector<PassPlan> plans;
     uint32_t nmax = 1, need_grid = 1;
-    int prc = plan_submission(S, D, T, sub, groups, plans, nmax, need_grid);
+    TableLayout TL;
+    int prc = plan_submission(S, D, T, sub, groups, plans, nmax, need_grid, TL);
     if (prc) return prc;
     if (first_pass == 0) {
         sub.passes.assign(groups.size(), PassRecord{});
@@ -447,19 +451,15 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         for (auto& v : sub.events) destroy_events(v);
         sub.events.assign(sub.timing ? groups.size() : 0, {});
     }
-    const TableLayout TL = table_layout(nmax);
     unsigned char* dtab = S.table.p;
     PassHeader* dhdr = (PassHeader*)dtab;
-    // the submission's status starts clear (a retry re-issues the failed
-    // passes with a clear status: the earlier ones succeeded)
-    FGC_CUDA(cudaMemsetAsync(&dhdr->status, 0, sizeof(unsigned int), stream));
 
     for (size_t g = first_pass; g < plans.size(); g++) {
         const PassPlan& P = plans[g];
         if (sub.cut && groups[g][0] == sub.cut) FGC_CUDA(cudaEventRecord(sub.at_cut, stream));
         PassRecord& rec = sub.passes[g];
         const uint32_t n = (uint32_t)P.views.size();
-        rec.in_off = g * TL.in_bytes();
+        rec.in_off = g * TL.total;
         rec.out_off = g * TL.out_bytes(nmax);
         rec.nbands = P.nbands;
         rec.band_rows = P.band_rows;
@@ -472,18 +472,29 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
 
         // ---- table upload
         unsigned char* hin = S.host_in.p + rec.in_off;
-        memcpy(hin, P.views.data(), (size_t)n * sizeof(ItemView));
-        uint32_t* hst = (uint32_t*)(hin + (TL.starts - TL.views));
+        memcpy(hin + TL.views, P.views.data(), (size_t)n * sizeof(ItemView));
+        uint32_t* hst = (uint32_t*)(hin + TL.starts);
         memcpy(hst, P.vtile.data(), (n + 1) * 4);
         memcpy(hst + (nmax + 1), P.stile.data(), (n + 1) * 4);
         memcpy(hst + 2 * (nmax + 1), P.blk.data(), (n + 1) * 4);
         memcpy(hst + 3 * (nmax + 1), P.band.data(), (n + 1) * 4);
-        FGC_CUDA(cudaMemcpyAsync(dtab + TL.views, hin, TL.in_bytes(), cudaMemcpyHostToDevice, stream));
-        FGC_CUDA(cudaMemsetAsync(&dhdr->c, 0, TL.out_bytes(n) - offsetof(PassHeader, c), stream));
         const uint64_t prim_cap0 = prim_capacity(P, S.clip_cap);
         const uint64_t rs_tiles = ceil_div(prim_cap0, 2048);
         const uint64_t ntiles = (uint64_t)P.stiles + P.scan_tiles + 4 + rs_tiles + 2;
-        FGC_CUDA(cudaMemsetAsync(S.tiles.p, 0, ntiles * 8, stream));
+        // The counters, per-draw outputs and look-back tiles start at zero, and
+        // so does the submission's status with its first pass (a retry re-issues
+        // the failed passes with a clear status: the earlier ones succeeded).
+        // They lie before the uploaded tables: one copy brings both where the
+        // zeros are few, else a memset comes first (three memsets and a copy took
+        // ~8 us of every draw's device time, one copy ~2).
+        const size_t from = g == first_pass ? offsetof(PassHeader, status) : offsetof(PassHeader, c);
+        if (TL.views <= kUploadZeros) {
+            memset(hin + from, 0, TL.views - from);
+            FGC_CUDA(cudaMemcpyAsync(dtab + from, hin + from, TL.total - from, cudaMemcpyHostToDevice, stream));
+        } else {
+            FGC_CUDA(cudaMemsetAsync(dtab + from, 0, TL.tiles + ntiles * 8 - from, stream));
+            FGC_CUDA(cudaMemcpyAsync(dtab + TL.views, hin + TL.views, TL.total - TL.views, cudaMemcpyHostToDevice, stream));
+        }
 
         const ItemView* items = (const ItemView*)(dtab + TL.views);
         const uint32_t* dst = (const uint32_t*)(dtab + TL.starts);
@@ -491,7 +502,7 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         ItemOut* iout = (ItemOut*)(dtab + TL.iout);
         PassCounters* dc = &dhdr->c;
         unsigned int* status = &dhdr->status;
-        unsigned long long* t_setup = S.tiles.p;
+        unsigned long long* t_setup = (unsigned long long*)(dtab + TL.tiles);
         unsigned long long* t_scan = t_setup + P.stiles + 2;
         unsigned long long* t_rscan = t_scan + P.scan_tiles + 2;
         const uint64_t prim_cap = prim_capacity(P, S.clip_cap);
