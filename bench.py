@@ -42,12 +42,12 @@ SS = 4
 
 # Algorithmic FP64 operations (add, subtract, multiply, divide, sqrt: one
 # each; compares not counted) of the reference's rasterize loop
-# (context.go:184-278) per event, for the Phong shader with an object colour,
-# no texture and SpecularPower 32 (shader.go:75-96, vertex.go:18-47).
+# (context.go:184-278) per event. Shading is not among them: the plain form's
+# colour bytes come from FP32 interval arithmetic wherever it decides them
+# (fgc_certshade.cuh, all but ~0.3 % of the fragments), the mixed form's from
+# FP32; the coverage and the depth are FP64 in both.
 FLOPS_PER_VISITED = 6        # b_k = w_k*ra (3), w_k += a_k (3)
 FLOPS_PER_COVERED = 6        # z (3 mul, 2 add), bz (1)
-FLOPS_PER_SHADED_PHONG = 119  # perspective 6, position 21, normal 31, Phong 61
-FLOPS_PER_SHADED_SOLID = 0
 # Triangle setup (drawClippedTriangle + rasterize prologue): NDC area per
 # triangle, edge setup per surviving primitive.
 FLOPS_SETUP_PER_TRIANGLE = 7
@@ -1006,8 +1006,7 @@ def main():
     names = list(_abi.STAGE_NAMES)
     dom = max(range(5), key=lambda i: stage[i])
     if names[dom] == "raster":
-        flops = (FLOPS_PER_VISITED * st.visited_pixels + FLOPS_PER_COVERED * st.covered_pixels
-                 + FLOPS_PER_SHADED_PHONG * st.shaded_fragments + st.shaded_fragments)
+        flops = FLOPS_PER_VISITED * st.visited_pixels + FLOPS_PER_COVERED * st.covered_pixels
     elif names[dom] == "setup":
         flops = FLOPS_SETUP_PER_TRIANGLE * st.elements + FLOPS_SETUP_PER_PRIM * st.primitives
     elif names[dom] == "vertex":

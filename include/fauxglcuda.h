@@ -325,9 +325,11 @@ typedef struct fgc_batch_item {
 typedef struct fgc_batch_tuning {
     int32_t band_pixels;          /* raster band size in pixels, whole rows (default 4096) */
     int32_t prims_per_bin_block;  /* primitives per binning block (default 4096)           */
-    int32_t fragment_cap;         /* fragment buffer of a raster CTA (default 1024)        */
+    int32_t fragment_cap;         /* fragment buffer of a raster CTA (default 1024; twice
+                                     that for passes of large primitives)                */
     int32_t use_graph;            /* 1: issue each submission as a CUDA graph              */
-    int32_t window;               /* raster pixels per thread and round for wide triangles (default 8) */
+    int32_t window;               /* 0-256; kept and reported, the raster stage sizes its
+                                     runs over wide triangles itself (default 8)         */
     int32_t reserved;
 } fgc_batch_tuning;
 int fgc_batch_create(fgc_batch** out);
