@@ -157,16 +157,15 @@ uint32_t pack_nrgba_host(const double c[4]) {
 namespace {
 void fill_cert(const StateView& sv, const ShaderView& shv, CertParams& C) {
     memset(&C, 0, sizeof(C));
-    if (sv.precision != FGC_PRECISION_PLAIN || shv.kind != FGC_SHADER_PHONG || shv.has_texture ||
-        shv.object_is_discard)
-        return;
+    if (sv.precision != FGC_PRECISION_PLAIN || shv.kind != FGC_SHADER_PHONG || shv.has_texture) return;
+    const bool vertex = shv.object_is_discard;
     const double alpha = shv.color[3];
-    if (!(alpha > 0 && alpha <= 1e6) || (sv.alpha_blend && alpha < 1)) return;
+    if (!vertex && (!(alpha > 0 && alpha <= 1e6) || (sv.alpha_blend && alpha < 1))) return;
     if (shv.pow_yi < 2 || shv.pow_yi > (uint64_t)kCertPowerMax) return;
     const double big = 1e6;  // products of the terms stay far inside FP32
     double l2 = 0, emax = 0;
     for (int k = 0; k < 3; k++) {
-        const double nonneg[4] = {shv.color[k], shv.ambient[k], shv.diffuse[k], shv.specular[k]};
+        const double nonneg[4] = {vertex ? 0.0 : shv.color[k], shv.ambient[k], shv.diffuse[k], shv.specular[k]};
         for (double v : nonneg)
             if (!(v >= 0 && v <= big) || (v > 0 && v < 1e-12)) return;
         if (!(std::fabs(shv.light[k]) <= big) || !(std::fabs(shv.eye[k]) <= big)) return;
@@ -174,7 +173,8 @@ void fill_cert(const StateView& sv, const ShaderView& shv, CertParams& C) {
         emax = std::max(emax, std::fabs(shv.eye[k]));
     }
     if (!(l2 >= 1e-6)) return;
-    C.on = 1;
+    C.on = vertex ? 0 : 1;
+    C.vertex = vertex ? 1 : 0;
     C.power = (int32_t)shv.pow_yi;
     C.powtol = (float)((C.power + 8) * 1.05 * kCertU);
     C.ln = (float)(std::sqrt(l2) * 1.0001);
@@ -191,7 +191,7 @@ void fill_cert(const StateView& sv, const ShaderView& shv, CertParams& C) {
         const double c = shv.color[k] * shv.ambient[k];
         unlit[k] = c < 1 ? c : 1;
     }
-    unlit[3] = alpha;
+    unlit[3] = vertex ? 1 : alpha;
     C.unlit = pack_nrgba_host(unlit);
 }
 }  // namespace

@@ -27,6 +27,9 @@
 //             monotone in its base: the interval's ends go through it.
 //   channel   colour * (ambient + diffuse N.L + specular s^p) * 255, all
 //             factors >= 0: 8 roundings, widened by 12u and 1e-6.
+//   vertex colours  sum w c / sum w from truncated FP64 weights, every term >=
+//             0: 13u; the channel is widened by 28u instead of 12u. Their alpha
+//             stays FP64.
 // A fragment with |N.L| <= eD is left to FP64 (the specular term switches on
 // there); N.L < -eD is the ambient colour, formed once per draw in FP64.
 //
@@ -46,7 +49,8 @@ constexpr int kCertPowerMax = 128;                // largest SpecularPower certi
 // A draw's shader parameters for cert_shade (filled on the host; `on` only
 // when every precondition of the bounds holds).
 struct CertParams {
-    int32_t on;
+    int32_t on;            // every fragment's colour is ObjectColor's
+    int32_t vertex;        // the vertices' colours take its place (on is 0)
     int32_t power;         // SpecularPower, an integer in [2, kCertPowerMax]
     uint32_t unlit;        // NRGBA of a fragment facing away from the light
     float light[3], ln;    // LightDirection and an upper bound on its length
@@ -107,6 +111,56 @@ FGC_HD uint32_t cs_u8(float v) {
 // gives a value above 2, which cert_shade rejects.
 FGC_HD float cert_bary(double b) { return f32_trunc_pos(fj_bits(b) & 0x7fffffffffffffffull); }
 
+// The shader from weights w* (their sum s; each within 4u), positions p* and
+// normals n* of the three vertices and the fragment's colour * 255 (within
+// tol - 12u). A fragment facing away from the light has the bytes of C.unlit,
+// or those of its own colour when it has one (vertex). alpha: the top byte.
+FGC_HD bool cert_light(const CertParams& C, float w0, float w1, float w2, float s, const float* p0, const float* p1,
+                       const float* p2, const float* n0, const float* n1, const float* n2, const float* col255,
+                       float tol, bool vertex, uint32_t alpha, uint32_t* out) {
+    float n[3], d[3];
+    for (int k = 0; k < 3; k++) n[k] = cs_fma(w2, n2[k], cs_fma(w1, n1[k], w0 * n0[k]));
+    const float rn = cs_rsqrt(cs_dot(n, n));
+    const float eN = 15.0f * kCertU * s * cs_max9(n0, n1, n2) * rn + 8.5f * kCertU;
+    if (!(eN < 0.01f && rn > 1e-18f)) return false;
+    for (int k = 0; k < 3; k++) n[k] = n[k] * rn;
+    const float nl = cs_dot(n, C.light);
+    const float eD = C.ln * (eN + 5.0f * kCertU) * 1.01f;
+    float nlo = 0.0f, nhi = 0.0f, lo = 0.0f, hi = 0.0f;
+    if (nl < -eD) {
+        if (!vertex) {
+            *out = C.unlit;
+            return true;
+        }
+    } else {
+        if (!(nl > eD)) return false;
+        for (int k = 0; k < 3; k++) d[k] = cs_fma(C.eye[k], s, -cs_fma(w2, p2[k], cs_fma(w1, p1[k], w0 * p0[k])));
+        const float rd = cs_rsqrt(cs_dot(d, d));
+        const float eC = 17.0f * kCertU * s * (C.emax + cs_max9(p0, p1, p2)) * rd + 8.5f * kCertU;
+        if (!(eC < 0.01f && rd > 1e-18f)) return false;
+        const float cl = cs_dot(d, C.light) * rd, cn = cs_dot(d, n) * rd;
+        const float sp = cs_fma(2.0f * nl, cn, -cl);
+        const float eS = C.ln * (4.0f * eN + 3.0f * eC + 24.0f * kCertU) * 1.05f;
+        hi = cs_pow(cs_max(sp + eS, 0.0f), C.power) * (1.0f + C.powtol);
+        lo = cs_pow(cs_max(sp - eS, 0.0f), C.power) * (1.0f - C.powtol);
+        nlo = nl - eD;
+        nhi = nl + eD;
+    }
+    uint32_t v = alpha;
+    bool same = true;
+    for (int k = 0; k < 3; k++) {
+        const float a = cs_fma(C.specular[k], lo, cs_fma(C.diffuse[k], nlo, C.ambient[k])) * col255[k];
+        const float b = cs_fma(C.specular[k], hi, cs_fma(C.diffuse[k], nhi, C.ambient[k])) * col255[k];
+        const uint32_t ia = cs_u8(a * (1.0f - tol) - 1e-6f);
+        const uint32_t ib = cs_u8(b * (1.0f + tol) + 1e-6f);
+        same = same && ia == ib && a <= b;  // a <= b is false for a NaN
+        v |= ia << (8 * k);
+    }
+    if (!same) return false;
+    *out = v;
+    return true;
+}
+
 // b*: truncated barycentrics, r*: FP32 1/W of the three vertices, p*/n*: their
 // FP32 positions and normals. Returns whether *out holds the fragment's bytes
 // (alpha in C.unlit's top byte).
@@ -119,42 +173,31 @@ FGC_HD bool cert_shade(const CertParams& C, float b0, float b1, float b2, float 
     const float w0 = b0 * r0, w1 = b1 * r1, w2 = b2 * r2;
     const float s = w0 + w1 + w2;
     if (!(s > 1e-18f)) return false;
-    float n[3], d[3];
-    for (int k = 0; k < 3; k++) n[k] = cs_fma(w2, n2[k], cs_fma(w1, n1[k], w0 * n0[k]));
-    const float rn = cs_rsqrt(cs_dot(n, n));
-    const float eN = 15.0f * kCertU * s * cs_max9(n0, n1, n2) * rn + 8.5f * kCertU;
-    if (!(eN < 0.01f && rn > 1e-18f)) return false;
-    for (int k = 0; k < 3; k++) n[k] = n[k] * rn;
-    const float nl = cs_dot(n, C.light);
-    const float eD = C.ln * (eN + 5.0f * kCertU) * 1.01f;
-    if (nl < -eD) {
-        *out = C.unlit;
-        return true;
-    }
-    if (!(nl > eD)) return false;
-    for (int k = 0; k < 3; k++) d[k] = cs_fma(C.eye[k], s, -cs_fma(w2, p2[k], cs_fma(w1, p1[k], w0 * p0[k])));
-    const float rd = cs_rsqrt(cs_dot(d, d));
-    const float eC = 17.0f * kCertU * s * (C.emax + cs_max9(p0, p1, p2)) * rd + 8.5f * kCertU;
-    if (!(eC < 0.01f && rd > 1e-18f)) return false;
-    const float cl = cs_dot(d, C.light) * rd, cn = cs_dot(d, n) * rd;
-    const float sp = cs_fma(2.0f * nl, cn, -cl);
-    const float eS = C.ln * (4.0f * eN + 3.0f * eC + 24.0f * kCertU) * 1.05f;
-    const float hi = cs_pow(cs_max(sp + eS, 0.0f), C.power) * (1.0f + C.powtol);
-    const float lo = cs_pow(cs_max(sp - eS, 0.0f), C.power) * (1.0f - C.powtol);
-    const float nlo = nl - eD, nhi = nl + eD;
-    uint32_t v = C.unlit & 0xff000000u;
-    bool same = true;
+    return cert_light(C, w0, w1, w2, s, p0, p1, p2, n0, n1, n2, C.color255, 12.0f * kCertU, false,
+                      C.unlit & 0xff000000u, out);
+}
+
+// The same with the vertices' colours c* (r, g, b) in place of ObjectColor, from
+// FP64 weights truncated to FP32 (2u each). The colour is sum w c / sum w, every
+// term >= 0: weights, colours and roundings 13u in all. alpha: its byte, from
+// FP64 (255 times a product of the weights' sum and its rounded reciprocal, which
+// decides between 254 and 255), in the top byte.
+FGC_HD bool cert_shade_vertex(const CertParams& C, float w0, float w1, float w2, const float* p0, const float* p1,
+                              const float* p2, const float* n0, const float* n1, const float* n2, const float* c0,
+                              const float* c1, const float* c2, uint32_t alpha, uint32_t* out) {
+    const float s = w0 + w1 + w2;
+    if (!(w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f && s > 1e-15f && s < 1e15f)) return false;
+    const float inv = 255.0f / s;
+    float col[3];
+    bool ok = true;
     for (int k = 0; k < 3; k++) {
-        const float a = cs_fma(C.specular[k], lo, cs_fma(C.diffuse[k], nlo, C.ambient[k])) * C.color255[k];
-        const float b = cs_fma(C.specular[k], hi, cs_fma(C.diffuse[k], nhi, C.ambient[k])) * C.color255[k];
-        const uint32_t ia = cs_u8(a * (1.0f - 12.0f * kCertU) - 1e-6f);
-        const uint32_t ib = cs_u8(b * (1.0f + 12.0f * kCertU) + 1e-6f);
-        same = same && ia == ib && a <= b;  // a <= b is false for a NaN
-        v |= ia << (8 * k);
+        // 0 or far from FP32's ends, where a bound relative to the value holds
+        ok = ok && (c0[k] == 0.0f || (c0[k] > 1e-12f && c0[k] < 1e6f)) &&
+             (c1[k] == 0.0f || (c1[k] > 1e-12f && c1[k] < 1e6f)) && (c2[k] == 0.0f || (c2[k] > 1e-12f && c2[k] < 1e6f));
+        col[k] = cs_fma(w2, c2[k], cs_fma(w1, c1[k], w0 * c0[k])) * inv;
     }
-    if (!same) return false;
-    *out = v;
-    return true;
+    if (!ok) return false;
+    return cert_light(C, w0, w1, w2, s, p0, p1, p2, n0, n1, n2, col, 28.0f * kCertU, true, alpha, out);
 }
 
 }  // namespace fgc

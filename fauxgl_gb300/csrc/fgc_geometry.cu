@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(64) clip_piece_kernel(GeomParams P) {
             if (mask) {
                 P.pool[pi] = PoolVertex{v[c].pos.x, v[c].pos.y, v[c].pos.z, v[c].nrm.x, v[c].nrm.y, v[c].nrm.z,
                                         v[c].tu, v[c].tv, v[c].col.x, v[c].col.y, v[c].col.z, v[c].col.w};
-                if (I.st.precision == FGC_PRECISION_MIXED || I.sh.cert.on)
+                if (I.st.precision == FGC_PRECISION_MIXED || I.sh.cert.on || I.sh.cert.vertex)
                     P.pool32[pi] = PoolVertex32{(float)v[c].pos.x, (float)v[c].pos.y, (float)v[c].pos.z,
                                                 (float)v[c].nrm.x, (float)v[c].nrm.y, (float)v[c].nrm.z,
                                                 (float)v[c].tu, (float)v[c].tv, (float)v[c].col.x,

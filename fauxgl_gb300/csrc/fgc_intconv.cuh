@@ -76,6 +76,13 @@ FGC_HD float f32_trunc_pos(uint64_t b) {
 #endif
 }
 
+// float32 of x truncated, the sign kept; the largest float32 for infinities and NaN.
+FGC_HD float f32_trunc(double x) {
+    const uint64_t b = fj_bits(x);
+    const float m = f32_trunc_pos(b & 0x7fffffffffffffffull);
+    return (b >> 63) ? -m : m;
+}
+
 // float64(v), exact for |v| < 2^53.
 FGC_HD double i2d_i(int64_t v) {
     if (v == 0) return 0.0;

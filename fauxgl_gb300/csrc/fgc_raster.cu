@@ -1088,6 +1088,46 @@ __device__ __forceinline__ bool certify(const RasterParams& P, const ItemView& I
                       out);
 }
 
+// A PhongShader fragment with vertex colours: its alpha in FP64 (16 of the
+// shader's ~100 FP64 instructions), its other bytes by cert_shade_vertex.
+// Returns its bytes, its flags above them, or 1 << 40; ~1 % of the fragments take
+// shade64, at once: their pixels' alphas differ, so that no mark could tell a
+// pending one (raster stage of a 1280x720 frame with vertex colours 196 -> 124
+// us).
+constexpr uint64_t kUncertain = 1ull << 40;
+__device__ __noinline__ uint64_t shade_vertex(const RasterParams& P, const ItemView& I, const RPrim& R, double b0,
+                                              double b1, double b2) {
+    D4 w = d4(__dmul_rn(b0, R.r0), __dmul_rn(b1, R.r1), __dmul_rn(b2, R.r2), 0.0);
+    const double s = __dadd_rn(__dadd_rn(w.x, w.y), w.z);
+    w.w = rcp_i(s);
+    const uint32_t v[3] = {R.v0, R.v1, R.v2};
+    float p[3][3], n[3][3], c[3][3];
+    double ca[3];
+    for (int k = 0; k < 3; k++) {
+        fetch_cert(P, I.mesh, v[k], p[k], n[k]);
+        if (v[k] & kPoolFlag) {
+            const PoolVertex32& q = P.pool32[v[k] & ~kPoolFlag];
+            c[k][0] = q.cr; c[k][1] = q.cg; c[k][2] = q.cb;
+            ca[k] = P.pool[v[k] & ~kPoolFlag].ca;
+        } else {
+            const float4 q = reinterpret_cast<const float4*>(I.mesh.col32)[v[k]];
+            c[k][0] = q.x; c[k][1] = q.y; c[k][2] = q.z;
+            ca[k] = I.mesh.col64[4 * (uint64_t)v[k] + 3];
+        }
+    }
+    const unsigned long long one = 0x3ff0000000000000ull;
+    // with alphas of 1 interp1's sum is s itself
+    const double alpha = dbits(ca[0]) == one && dbits(ca[1]) == one && dbits(ca[2]) == one
+                             ? __dmul_rn(s, w.w)
+                             : interp1(ca[0], ca[1], ca[2], w);
+    uint32_t out = 0;
+    if (dzero(alpha) ||  // a fragment of zeros is discarded
+        !cert_shade_vertex(I.sh.cert, f32_trunc(w.x), f32_trunc(w.y), f32_trunc(w.z), p[0], p[1], p[2], n[0], n[1],
+                           n[2], c[0], c[1], c[2], nrgba_pack_i(0.0, 0.0, 0.0, alpha) & 0xff000000u, &out))
+        return kUncertain;
+    return out | (I.st.alpha_blend && dlt1(alpha) ? (uint64_t)kFragBlend << 32 : 0);
+}
+
 // A pixel whose colour is pending holds mark + entry: the draw's colours all
 // have the alpha byte of `unlit`, a mark another one, so a pixel that no longer
 // holds an entry's mark was taken by a later fragment.
@@ -1140,6 +1180,14 @@ __device__ __forceinline__ void shade_fragment(const RasterParams& P, const Item
     }
     uint32_t packed;
     double c[4];
+    if (PREC == FGC_PRECISION_PLAIN && I.sh.cert.vertex && I.mesh.col32 && !P.dbg) {
+        const uint64_t v = shade_vertex(P, I, R, S.bd[f], S.bd[f + S.fcap], S.bd[f + 2 * S.fcap]);
+        if (v != kUncertain) {
+            S.col(f) = (uint32_t)v;
+            S.fflag[f] = (uint8_t)(v >> 32);
+            return;
+        }
+    }
     if (PREC == FGC_PRECISION_PLAIN && !S.exact) {  // SolidColorShader reads no barycentric
         for (int k = 0; k < 4; k++) c[k] = I.sh.color[k];
         fl = (uint8_t)I.sh.solid_flags;

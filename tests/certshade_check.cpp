@@ -55,7 +55,7 @@ static double go_pow(double x, int p) {
 int main(int argc, char** argv) {
     const long cases = argc > 1 ? atol(argv[1]) : 100000;
     const int powers[] = {2, 3, 7, 32, 50, 64, 128};
-    long certified = 0, ordinary = 0, ordinary_cert = 0;
+    long certified = 0, ordinary = 0, ordinary_cert = 0, vertex_cert = 0;
     for (long it = 0; it < cases; it++) {
         const int form = (int)(next64() % 8);
         fgc::CertParams C;
@@ -176,14 +176,40 @@ int main(int argc, char** argv) {
             printf("case %ld form %d power %d: %08x, FP64 %08x\n", it, form, C.power, got, want);
             return 1;
         }
+        // the same fragment with vertex colours
+        double vc[3][3];
+        float vf[3][3];
+        uint32_t wantv = 0x7b000000u;
+        const uint64_t kind = next64();
+        for (int v = 0; v < 3; v++)
+            for (int k = 0; k < 3; k++) {
+                vc[v][k] = kind & 1 ? (double)(next64() % 256) / 255.0 : uni() * 1.5;
+                if (kind % 8 == 2 && v) vc[v][k] = vc[0][k];
+                if (kind % 64 == 4) vc[v][k] = (next64() & 1) ? 0.0 : -uni();
+                vf[v][k] = (float)vc[v][k];
+            }
+        for (int k = 0; k < 3; k++) {
+            const double i = (((0 + vc[0][k] * w[0]) + vc[1][k] * w[1]) + vc[2][k] * w[2]) * w[3];
+            const double v = i * light;
+            wantv |= u8(v < 1 ? v : v == v ? 1 : v) << (8 * k);
+        }
+        uint32_t gotv = 0;
+        const bool okv = fgc::cert_shade_vertex(C, fgc::f32_trunc(w[0]), fgc::f32_trunc(w[1]), fgc::f32_trunc(w[2]),
+                                                pf[0], pf[1], pf[2], nf[0], nf[1], nf[2], vf[0], vf[1], vf[2],
+                                                0x7b000000u, &gotv);
+        if (okv && gotv != wantv) {
+            printf("vertex colours, case %ld form %d power %d: %08x, FP64 %08x\n", it, form, C.power, gotv, wantv);
+            return 1;
+        }
         certified += ok;
         if (form == 0 || form == 1) {
             ordinary++;
             ordinary_cert += ok;
+            vertex_cert += okv;
         }
     }
-    if (ordinary_cert < 0.95 * ordinary) {
-        printf("only %ld of %ld ordinary fragments certified\n", ordinary_cert, ordinary);
+    if (ordinary_cert < 0.95 * ordinary || vertex_cert < 0.9 * ordinary) {
+        printf("only %ld (vertex colours %ld) of %ld ordinary fragments certified\n", ordinary_cert, vertex_cert, ordinary);
         return 1;
     }
     printf("ok %.5f of all, %.5f of ordinary\n", (double)certified / cases, (double)ordinary_cert / ordinary);

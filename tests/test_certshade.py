@@ -68,3 +68,45 @@ def test_frames_match_oracle(gpu_lib, name, size, detail):
         assert tuple(info) == ref.draw(mesh, ctx.state(), ctx.shader_struct())
     assert np.array_equal(ctx.Image(), ref.color())
     assert np.array_equal(ctx.DepthBuffer.view(np.uint64), ref.depth().view(np.uint64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("blend", [True, False])
+@pytest.mark.parametrize("colors", ["opaque", "alphas", "zeros", "wild", "boundary"])
+@pytest.mark.parametrize("size,detail", [((97, 61), 3), ((640, 97), 2), ((1500, 40), 5)])
+def test_vertex_colors_match_oracle(gpu_lib, colors, blend, size, detail):
+    from fauxgl_gb300 import scenes
+    from fauxgl_gb300.context import CullNone, NewContext
+    from fauxgl_gb300.mesh import Mesh
+    from fauxgl_gb300.shader import NewPhongShader
+    from fauxgl_gb300.shapes import sphere_positions
+    from oracle import oracle as O
+
+    pos = scenes.displace(sphere_positions(detail), 5)
+    n = len(pos)
+    rng = np.random.RandomState(2)
+    col = rng.uniform(0, 1, (n, 3, 4))
+    col[..., 3] = 1.0
+    if colors == "alphas":
+        col[..., 3] = rng.choice([0.0, 0.3, 1.0, 1.5], (n, 3))
+    elif colors == "zeros":
+        col[rng.uniform(size=n) < 0.5] = 0.0
+    elif colors == "wild":
+        col[..., :3] = rng.choice([-0.5, 0.0, 1e-20, 1.0, 3.0, 1e9], (n, 3, 3))
+    elif colors == "boundary":  # whole faces of k / 255 steps
+        col[..., :3] = rng.randint(0, 256, (n, 1, 3)) / 255.0
+    mesh = Mesh(pos, pos, None, col)
+    w, h = size
+    ctx = NewContext(w, h)
+    ctx.Cull = CullNone
+    ctx.AlphaBlend = blend
+    ctx.ClearColorBufferWith(scenes.BACKGROUND)
+    eye = scenes.EYE
+    ctx.Shader = NewPhongShader(scenes.camera_matrix(w, h), scenes.LIGHT, eye)
+    ref = O.OracleContext(w, h)
+    ref.clear_color(scenes.BACKGROUND)
+    for draw in range(2):
+        info = ctx.DrawMesh(mesh)
+        assert tuple(info) == ref.draw(mesh, ctx.state(), ctx.shader_struct())
+    assert np.array_equal(ctx.Image(), ref.color())
+    assert np.array_equal(ctx.DepthBuffer.view(np.uint64), ref.depth().view(np.uint64))
