@@ -24,13 +24,13 @@ def test_texture_coordinates(gpu_lib, coords, alpha, size):
         im[..., 3] = 255
     n = 40
     pos = rng.uniform(-0.95, 0.95, (n, 3, 3))
-    tex = rng.uniform(0, 1, (n, 3, 3))
+    tex = rng.uniform(0, 1, (n, 3, 2))
     if coords == "outside":
-        tex = rng.uniform(-2.5, 3.5, (n, 3, 3))
+        tex = rng.uniform(-2.5, 3.5, (n, 3, 2))
     elif coords == "corners":
-        tex = rng.randint(-1, 3, (n, 3, 3)).astype(float)
+        tex = rng.randint(-1, 3, (n, 3, 2)).astype(float)
     elif coords == "texels":
-        tex = np.broadcast_to(rng.randint(0, 3, (n, 1, 3)) / np.array([max(w - 1, 1), max(h - 1, 1), 1.0]), (n, 3, 3)).copy()
+        tex = np.broadcast_to(rng.randint(0, 3, (n, 1, 2)) / np.array([max(w - 1, 1), max(h - 1, 1)]), (n, 3, 2)).copy()
     mesh = Mesh(pos, np.ones_like(pos), tex)
     ctx = NewContext(70, 50)
     ctx.Cull = CullNone
