@@ -30,6 +30,13 @@
 //   vertex colours  sum w c / sum w from truncated FP64 weights, every term >=
 //             0: 13u; the channel is widened by 28u instead of 12u. Their alpha
 //             stays FP64.
+// The bounds are relative, so they hold where nothing that matters nears the
+// ends of FP32's range. A fragment is therefore left to FP64
+//   - when n or d is not between 1e-15 and 1e18 long: n.n and d.d of a shorter
+//     vector are subnormal and lose bits (normals need not be unit vectors);
+//   - when the light reaches 1e14: a weight below FP32's normal range is off by
+//     up to 1.4e-45, a vertex colour by 3.6e-22 (weights from 1e-15, colours to
+//     1e6), which the light may multiply up to the 1e-6 that a channel is widened.
 // A fragment with |N.L| <= eD is left to FP64 (the specular term switches on
 // there); N.L < -eD is the ambient colour, formed once per draw in FP64.
 //
@@ -122,7 +129,7 @@ FGC_HD bool cert_light(const CertParams& C, float w0, float w1, float w2, float 
     for (int k = 0; k < 3; k++) n[k] = cs_fma(w2, n2[k], cs_fma(w1, n1[k], w0 * n0[k]));
     const float rn = cs_rsqrt(cs_dot(n, n));
     const float eN = 15.0f * kCertU * s * cs_max9(n0, n1, n2) * rn + 8.5f * kCertU;
-    if (!(eN < 0.01f && rn > 1e-18f)) return false;
+    if (!(eN < 0.01f && rn > 1e-18f && rn < 1e15f)) return false;
     for (int k = 0; k < 3; k++) n[k] = n[k] * rn;
     const float nl = cs_dot(n, C.light);
     const float eD = C.ln * (eN + 5.0f * kCertU) * 1.01f;
@@ -137,7 +144,7 @@ FGC_HD bool cert_light(const CertParams& C, float w0, float w1, float w2, float 
         for (int k = 0; k < 3; k++) d[k] = cs_fma(C.eye[k], s, -cs_fma(w2, p2[k], cs_fma(w1, p1[k], w0 * p0[k])));
         const float rd = cs_rsqrt(cs_dot(d, d));
         const float eC = 17.0f * kCertU * s * (C.emax + cs_max9(p0, p1, p2)) * rd + 8.5f * kCertU;
-        if (!(eC < 0.01f && rd > 1e-18f)) return false;
+        if (!(eC < 0.01f && rd > 1e-18f && rd < 1e15f)) return false;
         const float cl = cs_dot(d, C.light) * rd, cn = cs_dot(d, n) * rd;
         const float sp = cs_fma(2.0f * nl, cn, -cl);
         const float eS = C.ln * (4.0f * eN + 3.0f * eC + 24.0f * kCertU) * 1.05f;
@@ -150,10 +157,11 @@ FGC_HD bool cert_light(const CertParams& C, float w0, float w1, float w2, float 
     bool same = true;
     for (int k = 0; k < 3; k++) {
         const float a = cs_fma(C.specular[k], lo, cs_fma(C.diffuse[k], nlo, C.ambient[k])) * col255[k];
-        const float b = cs_fma(C.specular[k], hi, cs_fma(C.diffuse[k], nhi, C.ambient[k])) * col255[k];
+        const float most = cs_fma(C.specular[k], hi, cs_fma(C.diffuse[k], nhi, C.ambient[k]));
+        const float b = most * col255[k];
         const uint32_t ia = cs_u8(a * (1.0f - tol) - 1e-6f);
         const uint32_t ib = cs_u8(b * (1.0f + tol) + 1e-6f);
-        same = same && ia == ib && a <= b;  // a <= b is false for a NaN
+        same = same && ia == ib && a <= b && most < 1e14f;  // a <= b is false for a NaN
         v |= ia << (8 * k);
     }
     if (!same) return false;
