@@ -265,7 +265,7 @@ struct PassCounters {
 struct PassTuning {
     int64_t band_pixels = 4096;         // pixels per band, rounded to whole rows
     int64_t prims_per_bin_block = 4096; // raster primitives per binning block
-    int frag_cap = 1024;                // upper bound of the raster fragment buffer
+    int frag_cap = 1024;                // raster fragment buffer at most, rounded down to a multiple of 8 (twice it for large primitives; 4096)
     int window = 8;                     // accepted and reported; the raster stage sizes its runs itself
 };
 

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "fgc_device.cuh"
+#include "fgc_rasterfit.cuh"
 #include "fgc_scan.cuh"
 
 namespace fgc {
@@ -315,54 +316,7 @@ __global__ void attrs_kernel(const double* cp, const double* nrm, uint64_t n, AP
 __global__ void f64_to_f32_kernel(const double* in, uint64_t n, float* out);
 __global__ void fp64_rate_kernel(double* out, double a, double b, int iters);
 
-// Pixel buckets of the raster kernel's per-chunk fragment lists: as many as a
-// band has pixels by default, so that only fragments of one pixel share a
-// list; fewer where a row is longer than that and pixels share buckets anyway,
-// which leaves 4 KB for fragments (7680 pixels a row: 2.68 -> 2.59 ms).
-constexpr int kRasterHeadsMin = 2048;
-constexpr int kRasterHeadsMax = 4096;
-
 // Rows of a band at most.
 constexpr int kBandRowsMax = 128;
-
-// (primitive, row) units a chunk of wide primitives holds: kSpanUnitsMax
-// (the span arrays then also hold the narrow walk's warp queues) unless
-// shared memory cannot hold it, else kSpanUnitsMin. A primitive with more rows in a band than a chunk holds
-// (wrap-around rows of a box beyond the frame's sides) is split over chunks.
-constexpr int kSpanUnitsMin = 128;
-constexpr int kSpanUnitsMax = 256;
-
-// Pixels of a band at most; a wider frame is refused. The largest band whose
-// depth fits shared memory beside 256 fragments with FP64 barycentrics.
-constexpr int kBandPixelsMax = 26028;
-
-// Direct rounds (a unit per thread each) a chunk may take before its fragments
-// are shaded and resolved; one for frames too wide to hold their units. A
-// wireframe overlay leaves 55 fragments of 250 units after the early depth
-// test, and the phases after the walk were 40 % of its time: raster stage 5.12
-// ms with one round, 4.73 with two, 4.61 with three or four; 1080p dense 280,
-// 270, 266, 290 us (four rounds' memory is the L1 cache's).
-constexpr int kChunkRounds = 3;
-
-// Dynamic shared memory of the raster kernel (layout in fgc_raster.cu), for
-// a fragment buffer of F with barycentrics of bsize bytes and su span units:
-// depth[L] f64, fragment z[F] f64 and b0/b1/b2[F] (later their colours), span
-// edge values[su] 3 x f64, fragment key[F] u32, unit primitive/row[rounds *
-// 256] u32, span x/count/offset[su] u32, bucket list heads[heads] u16, list
-// links[F] u16, flags[F] u8. The colour buffer is not staged: the band's pixels
-// are read and written in global memory by the CTA that owns them.
-__host__ __device__ inline size_t raster_smem_bytes(int64_t L, int F, int su, int heads, int bsize, int rounds) {
-    size_t b = 0;
-    b += (size_t)L * 8;
-    b += (size_t)F * (8 + 3 * bsize);
-    b += (size_t)su * 8 * 3;
-    b += (size_t)F * 4;
-    b += (size_t)rounds * 256 * 4 * 2;
-    b += (size_t)su * 4 * 3;
-    b += (size_t)heads * 2;
-    b += (size_t)F * 2;
-    b += (size_t)F;
-    return (b + 15) & ~(size_t)15;
-}
 
 }  // namespace fgc

@@ -77,13 +77,9 @@ struct PassPlan {
     bool any_tri = false, any_line = false, debug_shaded = false;
     int32_t Lmax = 1, band_rows = 1, Rmax = 1;
     int precision = FGC_PRECISION_PLAIN;
-    int F = 0;
-    int su = kSpanUnitsMin;
-    int heads = kRasterHeadsMax;
-    int rounds = kChunkRounds;
+    RasterFit fit = {0, kSpanUnitsMin, kRasterHeadsMax, kChunkRounds, 0};
     int bsize = 4;               // bytes of a fragment's barycentric (8: some draw is shaded in FP64 throughout)
     bool cert = false;           // certified shading (some draw of the plain form takes it)
-    size_t smem = 0;
     int bin_warps = 1;
     uint32_t scan_tiles = 1;
     bool row_table = false;      // some draw uses the row-start table
@@ -123,45 +119,12 @@ std::vector<std::vector<uint32_t>> split_passes(const std::vector<PassItem>& ite
     return out;
 }
 
-int fit_fragments(const DevLimits& D, const PassTuning& T, int precision, int32_t Lmax, int bsize, bool large, int& F, int& su,
-                  int& heads, int& rounds, size_t& smem) {
-    const int stat = D.raster_static[precision == FGC_PRECISION_MIXED ? 1 : 0];
+int fit_fragments(const DevLimits& D, const PassTuning& T, PassPlan& P) {
+    const int stat = D.raster_static[P.precision == FGC_PRECISION_MIXED ? 1 : 0];
     const long two_cta = (long)D.smem_per_sm / 2 - D.smem_reserved_per_block - stat;
     const long one_cta = (long)D.smem_per_block_optin - stat;
-    // primitives of several pixels fill a larger buffer in one round of units
-    // (kRowTablePixelsPerElement); small ones do not, and its memory is then
-    // better left to the L1 cache (raster stage at twice the cap: 48 mixed
-    // thumbnails 2.33 -> 2.13 ms, a close-up 231 -> 218 us; a dense 1080p frame at
-    // 1.5 times 295 -> 315 us)
-    F = std::max(256, std::min(large ? 2 * T.frag_cap : T.frag_cap, 4096));
-    heads = Lmax > kRasterHeadsMax ? kRasterHeadsMin : kRasterHeadsMax;
-    rounds = kChunkRounds;
-    // the larger span arrays first: they also hold the warp queues of the
-    // narrow walk, which needs one 32-entry queue per warp (kSpanUnitsMax =
-    // the CTA's threads) and is worth more than a larger fragment buffer
-    su = kSpanUnitsMax;
-    smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
-    // two CTAs per SM (the register budget allows two) when a smaller
-    // fragment buffer makes them fit
-    while ((long)smem > two_cta && F > 512) {
-        F -= 128;
-        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
-    }
-    while ((long)smem > one_cta && F > 256) {
-        F /= 2;
-        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
-    }
-    if ((long)smem > one_cta) {
-        heads = kRasterHeadsMin;
-        rounds = 1;
-        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
-    }
-    if ((long)smem > one_cta) {
-        // the smaller span arrays (narrow rows then walk thread by thread)
-        su = kSpanUnitsMin;
-        smem = raster_smem_bytes(Lmax, F, su, heads, bsize, rounds);
-    }
-    if (Lmax > kBandPixelsMax || (long)smem > one_cta) return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
+    if (!fit_raster(two_cta, one_cta, T.frag_cap, P.Lmax, P.bsize, P.row_table, P.fit))
+        return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
     return FGC_OK;
 }
 
@@ -287,7 +250,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     P.band[n] = P.nbands;
     if (P.nmat >= 0xFFFFFFFFull) return fail(FGC_ERR_UNSUPPORTED, "pass too large for its bin matrix");
     P.scan_tiles = (uint32_t)ceil_div(P.nmat, 2048);
-    int rc = fit_fragments(D, T, P.precision, P.Lmax, P.bsize, P.row_table, P.F, P.su, P.heads, P.rounds, P.smem);
+    int rc = fit_fragments(D, T, P);
     if (rc) return rc;
     const int warps = (int)std::min<int64_t>(8, (96 * 1024) / ((int64_t)P.max_nbands * 4));
     if (warps < 1) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands for binning");
@@ -416,11 +379,11 @@ int plan_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, con
     FGC_CUDA(S.host_out.ensure(TL.out_bytes(nmax) * plans.size()));
     size_t need_pend = 0;
     for (const PassPlan& P : plans)
-        if (P.cert) need_pend = std::max(need_pend, (size_t)need_grid * pend_capacity(P.F));
+        if (P.cert) need_pend = std::max(need_pend, (size_t)need_grid * pend_capacity(P.fit.F));
     if (need_pend) FGC_CUDA(S.pend.ensure(need_pend));
     if (need_dbg) {
         size_t most = 0;
-        for (const PassPlan& P : plans) most = std::max(most, (size_t)need_grid * P.F * 4);
+        for (const PassPlan& P : plans) most = std::max(most, (size_t)need_grid * P.fit.F * 4);
         FGC_CUDA(S.dbg.ensure(most));
     }
     return FGC_OK;
@@ -691,14 +654,14 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.off = S.off.p;
         rp.nmat = P.nmat;
         rp.pair_total = &dc->pair_total;
-        rp.F = P.F;
+        rp.F = P.fit.F;
         rp.bsize = P.bsize;
-        rp.heads = P.heads;
-        rp.rounds = P.rounds;
+        rp.heads = P.fit.heads;
+        rp.rounds = P.fit.rounds;
         rp.Lmax = P.Lmax;
-        rp.su = P.su;
+        rp.su = P.fit.su;
         rp.pend = P.cert ? S.pend.p : nullptr;
-        rp.pend_cap = pend_capacity(P.F);
+        rp.pend_cap = pend_capacity(P.fit.F);
         rp.pool = S.pool.p;
         rp.pool32 = S.pool32.p;
         rp.rf = S.rf.p;
@@ -708,13 +671,13 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.status = status;
         rp.dbg = P.debug_shaded ? S.dbg.p : nullptr;
         const void* kfn = raster_kernel_ptr(P.precision);
-        FGC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+        FGC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.fit.smem));
         int per_sm = 0;
-        FGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kRasterThreads, P.smem));
+        FGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kRasterThreads, P.fit.smem));
         if (per_sm < 1) return fail(FGC_ERR_UNSUPPORTED, "raster kernel does not fit on an SM");
         int rgrid = (int)std::min<uint64_t>((uint64_t)per_sm * D.sms, P.nbands);
         if (P.debug_shaded || P.cert) rgrid = std::min<int>(rgrid, (int)need_grid);
-        FGC_CUDA(launch_raster(P.precision, rgrid, kRasterThreads, P.smem, stream, rp));
+        FGC_CUDA(launch_raster(P.precision, rgrid, kRasterThreads, P.fit.smem, stream, rp));
         rec.launches++;
         mark(evs, stream);
 

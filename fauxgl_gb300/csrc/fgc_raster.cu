@@ -38,24 +38,7 @@
 namespace fgc {
 
 constexpr int kRT = 256;  // threads per raster CTA
-struct RasterSmem {
-    double* depth;   // [L]
-    double* fz;      // [F]
-    float* bf;       // [3][F] barycentrics for FP32 shading; or, the same memory,
-    double* bd;      // [3][F] for FP64 shading of every fragment (exact)
-    int fcap;        // F
-    uint32_t* fkey;  // [F] (pixel << 16) | unit
-    double* uw0;     // [su] unit -> edge values at its first covered in-band pixel
-    double* uw1;
-    double* uw2;
-    uint32_t* uprim; // [P.rounds * kRT] unit -> primitive
-    int32_t* urow;   // [P.rounds * kRT] unit -> row y
-    int32_t* ux;     // [su] unit -> first covered in-band x
-    uint32_t* ucnt;  // [su] unit -> covered in-band pixels
-    uint32_t* ufrag; // [su] unit -> first fragment offset in the chunk
-    unsigned short* head;  // [kHeads] per pixel bucket: last fragment of its list (0xFFFF: none)
-    unsigned short* nxt;   // [F] per fragment: the previous fragment in its bucket
-    uint8_t* fflag;  // [F] discard / blend / pending flags
+struct RasterSmem : RasterArrays {
     PendFrag* pend;  // the CTA's fragments whose pixel colour is formed in FP64 later (global), or null
     uint32_t* npend; // entries of pend
     uint32_t mark;   // colour word of a pixel whose colour is pending, entry 0
@@ -1423,28 +1406,8 @@ __global__ void __launch_bounds__(kRT, 2) raster_kernel(RasterParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int F = P.F;
     RasterSmem S;
-    {
-        unsigned char* q = smem_raw;
-        S.depth = (double*)q; q += (size_t)P.Lmax * 8;
-        S.fz = (double*)q; q += (size_t)F * 8;
-        S.bf = (float*)q;
-        S.bd = (double*)q;
-        q += (size_t)F * 3 * P.bsize;
-        S.fcap = F;
-        S.uw0 = (double*)q; q += (size_t)P.su * 8;
-        S.uw1 = (double*)q; q += (size_t)P.su * 8;
-        S.uw2 = (double*)q; q += (size_t)P.su * 8;
-        S.fkey = (uint32_t*)q; q += (size_t)F * 4;
-        S.uprim = (uint32_t*)q; q += (size_t)P.rounds * kRT * 4;
-        S.urow = (int32_t*)q; q += (size_t)P.rounds * kRT * 4;
-        S.ux = (int32_t*)q; q += (size_t)P.su * 4;
-        S.ucnt = (uint32_t*)q; q += (size_t)P.su * 4;
-        S.ufrag = (uint32_t*)q; q += (size_t)P.su * 4;
-        S.head = (unsigned short*)q; q += (size_t)P.heads * 2;
-        S.hmask = (uint32_t)P.heads - 1;
-        S.nxt = (unsigned short*)q; q += (size_t)F * 2;
-        S.fflag = (uint8_t*)q;
-    }
+    place_raster(S, smem_raw, P.Lmax, F, P.su, P.heads, P.bsize, P.rounds);
+    S.hmask = (uint32_t)P.heads - 1;
     __shared__ uint32_t s_band, s_item, s_nfrag, s_conflict, s_nprim, s_nunit, s_ftotal, s_mode, s_bsum, s_ratio, s_split,
         s_rank, s_npend, s_fresh, s_held;
     __shared__ uint64_t s_warp[kRT / 32 + 1];

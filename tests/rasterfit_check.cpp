@@ -1,0 +1,52 @@
+// Goes through fit_raster and place_raster (fauxgl_gb300/csrc/fgc_rasterfit.cuh)
+// for every fragment cap, bands of many widths, both barycentric sizes and both
+// kinds of passes: every array must start on a multiple of its element's size and
+// the whole must fit. Prints "ok <cases>" or the first fault.
+// Build: g++ -O2 -std=c++17 rasterfit_check.cpp
+#include <cstdio>
+
+#include "../fauxgl_gb300/csrc/fgc_rasterfit.cuh"
+
+using namespace fgc;
+
+alignas(16) static unsigned char base[1 << 20];
+
+int main() {
+    const long per_sm = 233472, optin = 232448, reserved = 1024;  // sm_103a
+    long cases = 0;
+    for (long stat : {928L, 1056L})
+        for (int i = 0; i < 4200; i++) {
+            const int cap = i < 4190 ? 256 + i : 0x7fffffff >> (i - 4190) % 3;
+            for (int64_t L = 1; L < 60000; L = L < 40 ? L + 1 : L + L / 9 + i % 7)
+                for (int bsize : {4, 8})
+                    for (bool large : {false, true}) {
+                        RasterFit f;
+                        if (!fit_raster(per_sm / 2 - reserved - stat, optin - stat, cap, L, bsize, large, f)) {
+                            if (L < 26000) {
+                                printf("cap %d L %lld: refused\n", cap, (long long)L);
+                                return 1;
+                            }
+                            continue;
+                        }
+                        RasterArrays a;
+                        const unsigned char* end = place_raster(a, base, (int)L, f.F, f.su, f.heads, bsize, f.rounds);
+                        const void* eight[] = {a.depth, a.fz, bsize == 8 ? (void*)a.bd : base, a.uw0, a.uw1, a.uw2};
+                        const void* four[] = {a.bf, a.fkey, a.uprim, a.urow, a.ux, a.ucnt, a.ufrag};
+                        const void* two[] = {a.head, a.nxt};
+                        const size_t bytes = (size_t)(end - base);
+                        bool good = f.F >= 128 && f.F <= 4096 && f.smem <= (size_t)(optin - stat) && bytes <= f.smem &&
+                                    f.smem - bytes < 16 && (f.su == kSpanUnitsMin || f.su == kSpanUnitsMax);
+                        for (const void* o : eight) good = good && ((const unsigned char*)o - base) % 8 == 0;
+                        for (const void* o : four) good = good && ((const unsigned char*)o - base) % 4 == 0;
+                        for (const void* o : two) good = good && ((const unsigned char*)o - base) % 2 == 0;
+                        if (!good) {
+                            printf("cap %d L %lld bsize %d large %d: F %d, span values at %ld, %zu bytes\n", cap,
+                                   (long long)L, bsize, large, f.F, (long)((unsigned char*)a.uw0 - base), bytes);
+                            return 1;
+                        }
+                        cases++;
+                    }
+        }
+    printf("ok %ld\n", cases);
+    return 0;
+}
