@@ -26,9 +26,18 @@ constexpr int kRasterHeadsMax = 4096;
 constexpr int kSpanUnitsMin = 128;
 constexpr int kSpanUnitsMax = 256;
 
-// Pixels of a band at most; a wider frame is refused. The largest band whose
-// depth fits shared memory beside 256 fragments with FP64 barycentrics.
-constexpr int kBandPixelsMax = 26028;
+// A band's depth (8 bytes a pixel) and 51 bytes for each of the smallest_buffer
+// fragments at most; a wider frame is refused. 26,028 pixels with the default
+// cap, up to 26,844 with a smaller one.
+constexpr int64_t kBandBytesMax = 8 * 26028 + 51 * 256;
+
+// The smallest fragment buffer that the widest frames lead a cap to.
+inline int smallest_buffer(int frag_cap) {
+    int F = std::max(256, std::min(frag_cap, 4096));
+    while (F > 512) F -= 128;
+    while (F > 256) F /= 2;
+    return F;
+}
 
 // Direct rounds (a unit per thread each) a chunk may take before its fragments
 // are shaded and resolved; one for frames too wide to hold their units. A
@@ -139,7 +148,11 @@ inline bool fit_raster(long two_cta, long one_cta, int frag_cap, int64_t L, int 
         f.su = kSpanUnitsMin;
         size();
     }
-    return L <= kBandPixelsMax && (long)f.smem <= one_cta;
+    if ((long)f.smem > one_cta) {
+        f.F = smallest_buffer(frag_cap) & ~7;
+        size();
+    }
+    return L * 8 + smallest_buffer(frag_cap) * 51 <= kBandBytesMax && (long)f.smem <= one_cta;
 }
 
 }  // namespace fgc

@@ -1,7 +1,9 @@
 // Goes through fit_raster and place_raster (fauxgl_gb300/csrc/fgc_rasterfit.cuh)
 // for every fragment cap, bands of many widths, both barycentric sizes and both
-// kinds of passes: every array must start on a multiple of its element's size and
-// the whole must fit. Prints "ok <cases>" or the first fault.
+// kinds of passes: every array must start on a multiple of its element's size, the
+// whole must fit, and the widths that are accepted are those that a buffer of 51
+// bytes a fragment beside 10,240 bytes has room for, the cap reduced in steps of
+// 128 above 512 and halved above 256. Prints "ok <cases>" or the first fault.
 // Build: g++ -O2 -std=c++17 rasterfit_check.cpp
 #include <cstdio>
 
@@ -17,17 +19,19 @@ int main() {
     for (long stat : {928L, 1056L})
         for (int i = 0; i < 4200; i++) {
             const int cap = i < 4190 ? 256 + i : 0x7fffffff >> (i - 4190) % 3;
-            for (int64_t L = 1; L < 60000; L = L < 40 ? L + 1 : L + L / 9 + i % 7)
+            for (int64_t L = 1; L < 60000; L = L < 40 ? L + 1 : L > 25000 && L < 27000 ? L + 13 + i % 7 : L + L / 9 + i % 7)
                 for (int bsize : {4, 8})
                     for (bool large : {false, true}) {
                         RasterFit f;
-                        if (!fit_raster(per_sm / 2 - reserved - stat, optin - stat, cap, L, bsize, large, f)) {
-                            if (L < 26000) {
-                                printf("cap %d L %lld: refused\n", cap, (long long)L);
-                                return 1;
-                            }
-                            continue;
+                        const bool fits = fit_raster(per_sm / 2 - reserved - stat, optin - stat, cap, L, bsize, large, f);
+                        int least = cap < 4096 ? cap : 4096;
+                        while (least > 512) least -= 128;
+                        while (least > 256) least /= 2;
+                        if (fits != (8 * L + 51 * least + 10240 <= 231520)) {
+                            printf("cap %d L %lld: %s\n", cap, (long long)L, fits ? "accepted" : "refused");
+                            return 1;
                         }
+                        if (!fits) continue;
                         RasterArrays a;
                         const unsigned char* end = place_raster(a, base, (int)L, f.F, f.su, f.heads, bsize, f.rounds);
                         const void* eight[] = {a.depth, a.fz, bsize == 8 ? (void*)a.bd : base, a.uw0, a.uw1, a.uw2};

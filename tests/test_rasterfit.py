@@ -56,3 +56,36 @@ def test_any_fragment_cap_matches_oracle(gpu_lib, cap, shader, w, h):
         assert np.array_equal(ctx.DepthBuffer.view(np.uint64), ref.depth().view(np.uint64))
         step = np.abs(ctx.Image().astype(int) - ref.color().astype(int)).max()
         assert step <= (1 if shader == "mixed" else 0)  # one step in the mixed form
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cap,widest", [(256, 26028), (257, 26844), (300, 26703), (1000, 26104), (1024, 26028)])
+def test_widest_frame_of_a_cap(gpu_lib, cap, widest):
+    from fauxgl_gb300 import scenes
+    from fauxgl_gb300._abi import FauxGLError
+    from fauxgl_gb300.batch import Batch
+    from fauxgl_gb300.context import CullNone, NewContext
+    from fauxgl_gb300.geom import Identity
+    from fauxgl_gb300.mesh import Mesh
+    from fauxgl_gb300.shader import NewPhongShader
+    from oracle import oracle as O
+
+    rng = np.random.RandomState(cap)
+    pos = rng.uniform(-0.95, 0.95, (200, 1, 3)) + rng.uniform(-1, 1, (200, 3, 3)) * np.array([2e-3, 0.9, 0.02])
+    pos[150:] = rng.uniform(-0.95, 0.95, (50, 3, 3))
+    mesh = Mesh(np.clip(pos, -0.99, 0.99), rng.normal(size=pos.shape), None, rng.uniform(0, 1, (200, 3, 4)))
+    for w in (widest, widest + 1):
+        ctx = NewContext(w, 2)
+        ctx.Cull = CullNone
+        ctx.Shader = NewPhongShader(Identity(), scenes.LIGHT, scenes.EYE)
+        batch = Batch()
+        batch.SetTuning(fragment_cap=cap)
+        batch.Add(ctx, mesh)
+        if w > widest:
+            with pytest.raises(FauxGLError):
+                batch.Render()
+            continue
+        ref = O.OracleContext(w, 2)
+        assert tuple(batch.Render()[0]) == ref.draw(mesh, ctx.state(), ctx.shader_struct())
+        assert np.array_equal(ctx.Image(), ref.color())
+        assert np.array_equal(ctx.DepthBuffer.view(np.uint64), ref.depth().view(np.uint64))
