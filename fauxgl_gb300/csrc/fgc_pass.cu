@@ -95,6 +95,10 @@ constexpr double kRowTablePixelsPerElement = 8.0;
 constexpr int64_t kBinPrimsMin = 16;
 constexpr uint64_t kBinBlocksMin = 32;
 
+// Dynamic shared memory of the binning kernels at most.
+constexpr int64_t kBinSmemMax = 96 * 1024;
+static_assert(kMaxBands * 4 <= kBinSmemMax, "a block's histogram of the bands");
+
 uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
 // Draws go to the current pass until one repeats a target context (its
@@ -252,7 +256,7 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
     P.scan_tiles = (uint32_t)ceil_div(P.nmat, 2048);
     int rc = fit_fragments(D, T, P);
     if (rc) return rc;
-    const int warps = (int)std::min<int64_t>(8, (96 * 1024) / ((int64_t)P.max_nbands * 4));
+    const int warps = (int)std::min<int64_t>(8, kBinSmemMax / ((int64_t)P.max_nbands * 4));
     if (warps < 1) return fail(FGC_ERR_UNSUPPORTED, "frame has too many bands for binning");
     P.bin_warps = warps;
     return FGC_OK;
@@ -582,8 +586,6 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         bp.status = status;
         bp.pnb = S.pnb.p;
         const size_t hist_smem = (size_t)P.max_nbands * 4;
-        if (hist_smem > 48 * 1024)
-            FGC_CUDA(cudaFuncSetAttribute(bin_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem));
         bin_count_kernel<<<P.nblk, 256, hist_smem, stream>>>(bp);
         FGC_CUDA(cudaGetLastError());
         ScanParams sp;
@@ -632,8 +634,6 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
             rec.launches++;
         }
         const size_t scat_smem = (size_t)P.bin_warps * P.max_nbands * 4;
-        if (scat_smem > 48 * 1024)
-            FGC_CUDA(cudaFuncSetAttribute(bin_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scat_smem));
         bin_scatter_kernel<<<P.nblk, P.bin_warps * 32, scat_smem, stream>>>(bp, P.bin_warps);
         FGC_CUDA(cudaGetLastError());
         if (P.row_table) FGC_CUDA(cudaStreamWaitEvent(stream, S.ev_join, 0));
@@ -671,7 +671,6 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
         rp.status = status;
         rp.dbg = P.debug_shaded ? S.dbg.p : nullptr;
         const void* kfn = raster_kernel_ptr(P.precision);
-        FGC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.fit.smem));
         int per_sm = 0;
         FGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kRasterThreads, P.fit.smem));
         if (per_sm < 1) return fail(FGC_ERR_UNSUPPORTED, "raster kernel does not fit on an SM");
@@ -766,7 +765,7 @@ int run_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, cons
 }
 
 // ---------------------------------------------------------------------------
-// Device limits (read once per device)
+// Device limits (read, and the kernels' set, once per device)
 // ---------------------------------------------------------------------------
 int dev_limits(int device, const DevLimits** out) {
     static std::mutex mu;
@@ -779,11 +778,19 @@ int dev_limits(int device, const DevLimits** out) {
         FGC_CUDA(cudaDeviceGetAttribute(&D.smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
         FGC_CUDA(cudaDeviceGetAttribute(&D.smem_per_block_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         FGC_CUDA(cudaDeviceGetAttribute(&D.smem_reserved_per_block, cudaDevAttrReservedSharedMemoryPerBlock, device));
+        // The kernels' limits are raised once and for all: set for each launch, a
+        // smaller pass of another thread lowered them in between, and the launch
+        // failed (bands, and with them the memory, differ from frame to frame).
+        const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
         for (int p = 0; p < 2; p++) {
+            const void* fn = raster_kernel_ptr(p == 0 ? FGC_PRECISION_PLAIN : FGC_PRECISION_MIXED);
             cudaFuncAttributes fa;
-            FGC_CUDA(cudaFuncGetAttributes(&fa, raster_kernel_ptr(p == 0 ? FGC_PRECISION_PLAIN : FGC_PRECISION_MIXED)));
+            FGC_CUDA(cudaFuncGetAttributes(&fa, fn));
             D.raster_static[p] = (int)fa.sharedSizeBytes;
+            FGC_CUDA(cudaFuncSetAttribute(fn, limit, D.smem_per_block_optin - D.raster_static[p]));
         }
+        FGC_CUDA(cudaFuncSetAttribute(bin_count_kernel, limit, (int)kBinSmemMax));
+        FGC_CUDA(cudaFuncSetAttribute(bin_scatter_kernel, limit, (int)kBinSmemMax));
         D.device = device;
     }
     *out = &D;
