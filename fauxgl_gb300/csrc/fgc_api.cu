@@ -84,8 +84,10 @@ cudaError_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, P->pool[kind], s);
-    if (e == cudaErrorMemoryAllocation) {  // with the other pools' spare memory
+    if (e == cudaErrorMemoryAllocation) {  // with the other pools' spare memory, once its frees have taken effect
         cudaGetLastError();
+        cudaStreamSynchronize(P->free_stream);
+        cudaStreamSynchronize(s);
         for (cudaMemPool_t pool : P->pool) cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, P->pool[kind], s);
     }
@@ -104,7 +106,7 @@ cudaError_t big_alloc(void** p, size_t bytes) {
         e = device_pool(&P);
     }
     if (e != cudaSuccess) return e;
-    cudaDeviceSynchronize();
+    cudaStreamSynchronize(P->free_stream);
     for (cudaMemPool_t pool : P->pool) cudaMemPoolTrimTo(pool, 0);
     return cudaMalloc(p, bytes);
 }
@@ -136,6 +138,21 @@ cudaStream_t free_stream() {
     std::lock_guard<std::mutex> lock(g_pool_mu);
     DevicePool* P = nullptr;
     return device_pool(&P) == cudaSuccess ? P->free_stream : nullptr;
+}
+
+std::shared_mutex& capture_mutex() {
+    static std::shared_mutex mu;
+    return mu;
+}
+
+void device_wait() {
+    std::unique_lock<std::shared_mutex> lock(capture_mutex());
+    if (cudaDeviceSynchronize() == cudaSuccess) return;
+    cudaGetLastError();
+    // a capture that is not the library's: cudaFree waits as well and is permitted
+    void* p = nullptr;
+    if (cudaMalloc(&p, 1) == cudaSuccess) cudaFree(p);
+    else cudaGetLastError();
 }
 
 uint32_t pack_nrgba_host(const double c[4]) {
@@ -698,7 +715,7 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
 int fgc_mesh_release(fgc_mesh* m) {
     if (!m) return FGC_OK;
     cudaSetDevice(m->device);
-    cudaDeviceSynchronize();
+    fgc::device_wait();
     delete m;
     return FGC_OK;
 }
@@ -726,7 +743,7 @@ int fgc_texture_upload(const uint16_t* rgba16, int32_t width, int32_t height, fg
     if (e == cudaSuccess) {
         fgc::texel_unit_kernel<<<fgc::grid_for(n, 256, 4096), 256>>>(t->texels.p, n, t->unit64.p);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     }
     if (e != cudaSuccess) {
         delete t;
@@ -739,7 +756,7 @@ int fgc_texture_upload(const uint16_t* rgba16, int32_t width, int32_t height, fg
 int fgc_texture_release(fgc_texture* t) {
     if (!t) return FGC_OK;
     cudaSetDevice(t->device);
-    cudaDeviceSynchronize();
+    fgc::device_wait();
     delete t;
     return FGC_OK;
 }
@@ -813,7 +830,7 @@ int fgc_depth_image(fgc_context* c, uint16_t* gray16) {
     FGC_CUDA(cudaSetDevice(c->device));
     int rc = apply_pending_clears(c);
     if (rc) return rc;
-    FGC_CUDA(c->lohi.ensure(2));
+    FGC_CUDA(c->lohi.ensure(2));  // one size each: they do not grow
     FGC_CUDA(c->gray.ensure((size_t)c->N));
     unsigned long long init[2] = {~0ull, 0ull};
     FGC_CUDA(cudaMemcpyAsync(c->lohi.p, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
@@ -837,7 +854,7 @@ int fgc_downsample(fgc_context* c, int32_t scale, uint8_t* out) {
     int rc = apply_pending_clears(c);
     if (rc) return rc;
     const uint64_t n = (uint64_t)(c->W / scale) * (uint64_t)(c->H / scale);
-    FGC_CUDA(c->ds.ensure(n));
+    FGC_CUDA(c->ds.ensure(n, c->stream));
     downsample_kernel<<<grid_for(n, 256, c->sms * 8), 256, 0, c->stream>>>(c->color.p, c->W, c->H, scale, c->ds.p);
     FGC_CUDA(cudaGetLastError());
     FGC_CUDA(cudaMemcpyAsync(out, c->ds.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -873,7 +890,7 @@ int fgc_read_shaded_color(fgc_context* c, double* rgba) {
 // ===========================================================================
 // DepthImage without device allocation.
 //
-// fgc_depth_image above grows c->lohi and c->gray with cudaMalloc the first
+// fgc_depth_image above allocates c->lohi and c->gray on the device the first
 // time it runs. Callers that may not let the library allocate device memory
 // once they are running (a service that reserves all its buffers before it
 // admits work, a host application that owns the GPU memory of its plugins)

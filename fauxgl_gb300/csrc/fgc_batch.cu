@@ -129,6 +129,22 @@ void release_contexts(fgc_batch* b) {
     b->contexts.clear();
 }
 
+// Wait for a submission that failed on the way: its draws and read-backs must
+// not outlive the call.
+void abandon(fgc_batch* b) {
+    abandon_submission(b->scratch, b->stream);
+    if (b->copy) cudaStreamSynchronize(b->copy);
+}
+
+// Issue the submission's passes from `from` on and its read-backs.
+int issue_passes_and_reads(fgc_batch* b, size_t from) {
+    const DevLimits* D = nullptr;
+    int rc = dev_limits(b->device, &D);
+    if (rc == FGC_OK) rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, from);
+    if (rc == FGC_OK) rc = enqueue_all_reads(b);
+    return rc;
+}
+
 // Issue the submission in b->sub (passes from the first) and its read-backs.
 int issue(fgc_batch* b) {
     const DevLimits* D = nullptr;
@@ -137,9 +153,7 @@ int issue(fgc_batch* b) {
     rc = prepare_submission(b->scratch, *D, b->tuning, b->sub);
     if (rc) return rc;
     if (!b->use_graph) {
-        rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, 0);
-        if (rc) return rc;
-        rc = enqueue_all_reads(b);
+        rc = issue_passes_and_reads(b, 0);
         if (rc) return rc;
         FGC_CUDA(cudaEventRecord(b->done, b->stream));
         return FGC_OK;
@@ -147,11 +161,14 @@ int issue(fgc_batch* b) {
     // Capture the submission and replay it as one graph launch; an
     // executable graph from an earlier submission is updated in place when
     // the new one has the same shape, otherwise instantiated anew.
-    FGC_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, 0);
-    if (rc == FGC_OK) rc = enqueue_all_reads(b);
     cudaGraph_t g = nullptr;
-    cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
+    cudaError_t ce;
+    {
+        std::shared_lock<std::shared_mutex> capturing(capture_mutex());
+        FGC_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+        rc = issue_passes_and_reads(b, 0);
+        ce = cudaStreamEndCapture(b->stream, &g);
+    }
     if (rc) {
         if (g) cudaGraphDestroy(g);
         return rc;
@@ -182,22 +199,17 @@ int issue(fgc_batch* b) {
 // Wait for the submission in flight, re-issue failed passes (and the
 // read-backs after them) until every pass has succeeded.
 int finish(fgc_batch* b) {
-    const DevLimits* D = nullptr;
-    int rc = dev_limits(b->device, &D);
-    if (rc) return rc;
     size_t from = 0;
     for (int attempt = 0; attempt < 8; attempt++) {
         FGC_CUDA(cudaStreamSynchronize(b->stream));
         size_t next = 0;
-        rc = collect_submission(b->scratch, b->sub, from, &next);
+        int rc = collect_submission(b->scratch, b->sub, from, &next);
         if (rc) return rc;
         if (next == b->sub.passes.size()) return FGC_OK;
         from = next;
         // a pass overflowed: it and the passes after it left their targets
         // untouched; run them again with the sizes the device measured
-        rc = issue_submission(b->scratch, b->stream, *D, b->tuning, b->sub, from);
-        if (rc) return rc;
-        rc = enqueue_all_reads(b);
+        rc = issue_passes_and_reads(b, from);
         if (rc) return rc;
     }
     return fail(FGC_ERR_DEVICE_LIMIT, "draw buffers kept overflowing");
@@ -284,6 +296,7 @@ int submit(fgc_batch* b, const fgc_batch_item* items, uint64_t n) {
     sub.reset();
     int rc = issue(b);
     if (rc) {
+        abandon(b);
         release_contexts(b);
         return rc;
     }
@@ -294,6 +307,7 @@ int submit(fgc_batch* b, const fgc_batch_item* items, uint64_t n) {
 int wait(fgc_batch* b, fgc_rasterize_info* infos) {
     if (!b->inflight) return fail(FGC_ERR_INVALID_ARGUMENT, "the batch has no submission in flight");
     int rc = finish(b);
+    if (rc) abandon(b);
     b->inflight = false;
     release_contexts(b);
     b->stats = b->sub.stats;
@@ -336,6 +350,7 @@ int fgc_batch_destroy(fgc_batch* b) {
         cudaSetDevice(b->device);
         if (b->inflight) wait(b, nullptr);
         cudaStreamSynchronize(b->stream);
+        if (b->copy) cudaStreamSynchronize(b->copy);
         if (b->exec) cudaGraphExecDestroy(b->exec);
         if (b->done) cudaEventDestroy(b->done);
         if (b->copied) cudaEventDestroy(b->copied);

@@ -17,6 +17,7 @@
 #include <cstddef>
 #include <cstring>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -59,10 +60,16 @@ void pool_free(void* p, cudaStream_t s);
 cudaError_t big_alloc(void** p, size_t bytes);
 // A stream of the device for one call (kept for later calls, at most eight)
 // and its return. free_stream: the stream on which memory outliving its call
-// is freed, after the device has been waited for.
+// is freed, once nothing uses it any more.
 cudaError_t take_stream(int device, cudaStream_t* s);
 void give_stream(int device, cudaStream_t s);
 cudaStream_t free_stream();
+// Waits for all work of the current device. While a thread captures a stream
+// cudaDeviceSynchronize is not permitted to any thread -- it breaks the capture
+// --, so batches hold capture_mutex shared while they capture, and this call
+// holds it alone.
+std::shared_mutex& capture_mutex();
+void device_wait();
 
 // n elements of pool memory in the order of stream s: a call's temporary (Kept
 // false: freed in that order as well) or an array of a mesh (Kept true).
@@ -99,8 +106,11 @@ using TempBuf = PoolBuf<T, false>;
 template <typename T>
 using MeshBuf = PoolBuf<T, true>;
 
-// A buffer that any stream may use: the device is waited for before it is
-// freed, and its allocation has taken effect before it is used.
+// A buffer that any stream may use: its allocation has taken effect before it
+// is used. Its owner sees to it that nothing uses it any more when it is
+// released or grows: contexts and batches wait for their streams, also where a
+// call fails, meshes and textures for the device. (Waiting for the device here
+// would break the graph capture of another thread, see device_wait.)
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
@@ -111,14 +121,18 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void release() {
         if (p) {
-            cudaDeviceSynchronize();
             if (cap * sizeof(T) >= kPoolBufMax) cudaFree(p);
             else pool_free(p, free_stream());
         }
         p = nullptr;
         cap = 0;
     }
-    // Make room for n elements (contents not preserved when it grows).
+    // Make room for n elements (contents not preserved when it grows); user: the
+    // stream whose work may use the buffer still.
+    cudaError_t ensure(size_t n, cudaStream_t user) {
+        if (n > cap && p) cudaStreamSynchronize(user);
+        return ensure(n);
+    }
     cudaError_t ensure(size_t n) {
         if (n <= cap && p) return cudaSuccess;
         release();
@@ -319,6 +333,7 @@ struct PassScratch {
     PassScratch(const PassScratch&) = delete;
     PassScratch& operator=(const PassScratch&) = delete;
     ~PassScratch() {
+        if (side) cudaStreamSynchronize(side);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (side) cudaStreamDestroy(side);
@@ -359,9 +374,11 @@ struct Submission {
 int prepare_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, const Submission& sub);
 // Split items into passes and issue passes [first_pass, end) on stream (no
 // host wait), each followed by the copy of its results. The submission's
-// status word is zeroed first.
+// status word is zeroed first. An issue that fails has been waited for.
 int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, const PassTuning& T,
                      Submission& sub, size_t first_pass);
+// Wait for what a failed issue has left running (nothing while capturing).
+void abandon_submission(PassScratch& S, cudaStream_t stream);
 // After the stream has drained: read the results of passes [from, end).
 // Sets *retry_from = passes.size() when they all succeeded; otherwise grows
 // the scratch limits and sets *retry_from to the first pass to re-issue.

@@ -403,8 +403,9 @@ int prepare_submission(PassScratch& S, const DevLimits& D, const PassTuning& T, 
     return plan_submission(S, D, T, sub, groups, plans, nmax, need_grid, TL);
 }
 
-int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, const PassTuning& T, Submission& sub,
-                     size_t first_pass) {
+namespace {
+int issue_passes(PassScratch& S, cudaStream_t stream, const DevLimits& D, const PassTuning& T, Submission& sub,
+                 size_t first_pass) {
     if (sub.items.empty()) return FGC_OK;
     std::vector<std::vector<uint32_t>> groups;
     std::vector<PassPlan> plans;
@@ -686,6 +687,22 @@ int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, co
     return FGC_OK;
 }
 
+}  // namespace
+
+int issue_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, const PassTuning& T, Submission& sub,
+                     size_t first_pass) {
+    const int rc = issue_passes(S, stream, D, T, sub, first_pass);
+    if (rc) abandon_submission(S, stream);
+    return rc;
+}
+
+void abandon_submission(PassScratch& S, cudaStream_t stream) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return;
+    cudaStreamSynchronize(stream);
+    if (S.side) cudaStreamSynchronize(S.side);
+}
+
 int collect_submission(PassScratch& S, Submission& sub, size_t from, size_t* retry_from) {
     *retry_from = sub.passes.size();
     fgc_stats& st = sub.stats;
@@ -754,6 +771,7 @@ int finish_submission(PassScratch& S, cudaStream_t stream, const DevLimits& D, c
         rc = issue_submission(S, stream, D, T, sub, from);
         if (rc) return rc;
     }
+    abandon_submission(S, stream);
     return fail(FGC_ERR_DEVICE_LIMIT, "draw buffers kept overflowing");
 }
 
