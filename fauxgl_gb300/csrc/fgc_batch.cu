@@ -109,9 +109,17 @@ uint32_t read_cut(const fgc_batch* b) {
     std::sort(targets.begin(), targets.end());
     if (std::adjacent_find(targets.begin(), targets.end()) != targets.end()) return 0;
     double us = 0;
-    for (const fgc_batch::ReadBack& r : b->reads)
-        us += 10.0 + (double)r.ctx->N * 4 / ((double)r.scale * r.scale) / 190e3;
+    std::vector<std::pair<const uint8_t*, const uint8_t*>> dst;
+    for (const fgc_batch::ReadBack& r : b->reads) {
+        const size_t bytes = (size_t)(r.ctx->W / r.scale) * (size_t)(r.ctx->H / r.scale) * 4;
+        us += 10.0 + (double)bytes / 190e3;
+        dst.emplace_back(r.dst, r.dst + bytes);
+    }
     if (us < kReadCutMin) return 0;
+    // where two frames are read to the same place the later one stays: in order
+    std::sort(dst.begin(), dst.end());
+    for (size_t i = 1; i < dst.size(); i++)
+        if (dst[i].first < dst[i - 1].second) return 0;
     uint64_t total = 0, sum = 0;
     for (const PassItem& p : items) total += (uint64_t)p.ctx->N;
     for (uint32_t i = 0; i < (uint32_t)items.size(); i++) {
