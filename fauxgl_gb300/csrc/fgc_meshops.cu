@@ -176,9 +176,12 @@ __global__ void group_sort_kernel(const uint32_t* start, const uint32_t* count, 
 // +1: the FP64 dot product of the normals behind a and b is at least thr, -1:
 // below it, 0: too near to tell. The FP32 dot product of rounded components is
 // within 6 * 2^-24 of the sum of its products' sizes; thr is rounded once.
+// Components below FP32's normal range are off by up to 2^-150 instead, times
+// the other normal's, which may be as long as 1e38.
 __device__ __forceinline__ int side_of(const APosNrm32& a, const APosNrm32& b, float thr) {
     const float x = a.nx * b.nx, y = a.ny * b.ny, z = a.nz * b.nz;
-    const float d = x + y + z - thr, e = 6e-7f * (fabsf(x) + fabsf(y) + fabsf(z) + fabsf(thr)) + 1e-35f;
+    const float sub = 1.4e-45f * (fabsf(a.nx) + fabsf(a.ny) + fabsf(a.nz) + fabsf(b.nx) + fabsf(b.ny) + fabsf(b.nz));
+    const float d = x + y + z - thr, e = 6e-7f * (fabsf(x) + fabsf(y) + fabsf(z) + fabsf(thr)) + sub + 1e-35f;
     return d > e ? 1 : d < -e ? -1 : 0;  // NaN and infinities: 0
 }
 
