@@ -23,7 +23,7 @@ def __getattr__(name):
     # The context layer needs the CUDA library; import it lazily so the host
     # helpers (scenes, meshes, matrices) are usable where it is not built.
     if name in ("Context", "NewContext", "RasterizeInfo", "FaceCW", "FaceCCW", "CullNone", "CullFront",
-                "CullBack", "PRECISION_PLAIN", "PRECISION_MIXED"):
+                "CullBack", "PRECISION_PLAIN", "PRECISION_MIXED", "TrimMemory"):
         from . import context
         return getattr(context, name)
     if name in ("LoadSTL", "DeviceMesh"):

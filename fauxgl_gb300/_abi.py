@@ -163,6 +163,7 @@ SIGNATURES = {
     "fgc_mesh_download": (_I, [_P, _D, _D, _D, _D]),
     "fgc_texture_upload": (_I, [ctypes.POINTER(ctypes.c_uint16), _I32, _I32, _PP]),
     "fgc_texture_release": (_I, [_P]),
+    "fgc_trim_memory": (_I, []),
     "fgc_draw_mesh": (_I, [_P, _P, _ST, _SH, _INFO]),
     "fgc_draw_triangles": (_I, [_P, _P, _U64, _U64, _ST, _SH, _INFO]),
     "fgc_draw_lines": (_I, [_P, _P, _U64, _U64, _ST, _SH, _INFO]),

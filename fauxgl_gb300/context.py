@@ -283,3 +283,9 @@ class Context:
 def NewContext(width, height):
     """context.go:60-81."""
     return Context(width, height)
+
+
+def TrimMemory():
+    """Give the device memory that the library keeps for later calls back to the
+    driver (no reference counterpart)."""
+    _abi.check(_abi.load_library().fgc_trim_memory())

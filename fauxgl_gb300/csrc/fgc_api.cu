@@ -42,6 +42,7 @@ struct DevicePool {
     cudaMemPool_t pool[kPoolKinds] = {};
     cudaStream_t free_stream = nullptr;
     std::vector<cudaStream_t> idle;
+    uint64_t live = 0;  // objects on the device
 };
 std::mutex g_pool_mu;
 DevicePool g_pools[kMaxDevices];
@@ -109,6 +110,36 @@ cudaError_t big_alloc(void** p, size_t bytes) {
     cudaStreamSynchronize(P->free_stream);
     for (cudaMemPool_t pool : P->pool) cudaMemPoolTrimTo(pool, 0);
     return cudaMalloc(p, bytes);
+}
+
+cudaError_t trim_pools(uint64_t keep) {
+    DevicePool* P = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        const cudaError_t e = device_pool(&P);
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = cudaStreamSynchronize(P->free_stream);
+    for (cudaMemPool_t pool : P->pool)
+        if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, keep);
+    return e;
+}
+
+void Live::on(int dev) {
+    if (dev < 0 || dev >= kMaxDevices) return;
+    device = dev;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    g_pools[dev].live++;
+}
+
+Live::~Live() {
+    if (device < 0) return;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (--g_pools[device].live != 0 || !g_pools[device].free_stream) return;
+    }
+    // the release that ends here has made the device current
+    if (trim_pools(kPoolIdle) != cudaSuccess) cudaGetLastError();
 }
 
 cudaError_t take_stream(int device, cudaStream_t* s) {
@@ -497,6 +528,7 @@ int fgc_context_create(int32_t width, int32_t height, fgc_context** out) {
     };
     cudaError_t e = cudaGetDevice(&c->device);
     if (e != cudaSuccess) return bail(fail(FGC_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e)));
+    c->live.on(c->device);
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(fail(FGC_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e)));
@@ -650,6 +682,7 @@ int fgc_mesh_upload(const double* tri_pos, const double* tri_nrm, const double* 
     int dev = 0;
     cudaGetDevice(&dev);
     m->device = dev;
+    m->live.on(dev);
     m->ntri = ntri;
     m->nline = nline;
     int sms = 1;
@@ -727,6 +760,11 @@ int fgc_mesh_counts(const fgc_mesh* m, uint64_t* ntri, uint64_t* nline) {
     return FGC_OK;
 }
 
+int fgc_trim_memory(void) {
+    FGC_CUDA(trim_pools(0));
+    return FGC_OK;
+}
+
 int fgc_texture_upload(const uint16_t* rgba16, int32_t width, int32_t height, fgc_texture** out) {
     if (!out || !rgba16) return fail(FGC_ERR_INVALID_ARGUMENT, "null argument");
     *out = nullptr;
@@ -734,6 +772,7 @@ int fgc_texture_upload(const uint16_t* rgba16, int32_t width, int32_t height, fg
     fgc_texture* t = new (std::nothrow) fgc_texture();
     if (!t) return fail(FGC_ERR_OUT_OF_MEMORY, "host allocation failed");
     cudaGetDevice(&t->device);
+    t->live.on(t->device);
     t->w = width;
     t->h = height;
     size_t n = (size_t)width * height;

@@ -12,6 +12,7 @@
 using namespace fgc;
 
 struct fgc_batch {
+    fgc::Live live;
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
@@ -347,6 +348,7 @@ int fgc_batch_create(fgc_batch** out) {
         return fail(FGC_ERR_CUDA, std::string("batch setup: ") + cudaGetErrorString(e));
     }
     b->stream = b->own_stream;
+    b->live.on(b->device);
     *out = b;
     return FGC_OK;
 }

@@ -44,10 +44,13 @@ int fail(int code, const std::string& msg);
 // into a new 1080p context, which allocates its scratch, takes 1.27 ms instead
 // of 2.36. Each pool keeps at most kPoolKeep bytes of freed memory (the driver
 // returns the rest when a stream synchronises), so that many resident meshes
-// or large frames do not take the temporaries' share. The pools are the
+// or large frames do not take the temporaries' share. When the library's last
+// object on the device is released they go back to kPoolIdle bytes, and
+// fgc_trim_memory gives back everything unused at any time. The pools are the
 // driver's, so threads and streams may use them together: memory freed on one
 // stream is handed to another only once that free has taken effect.
 constexpr uint64_t kPoolKeep = 1ull << 30;
+constexpr uint64_t kPoolIdle = 128ull << 20;
 // Frame and scratch buffers from this size on are allocations of their own: a
 // pool grows in small pieces, and one that has to grow by several GB takes
 // longer than cudaMalloc (first pass over a 7680x4320 frame with a wireframe
@@ -58,6 +61,19 @@ cudaError_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s);
 void pool_free(void* p, cudaStream_t s);
 // cudaMalloc, the pools' kept memory given back first where it is in the way.
 cudaError_t big_alloc(void** p, size_t bytes);
+// The current device's pools reduced to `keep` bytes each, as far as their
+// memory is unused.
+cudaError_t trim_pools(uint64_t keep);
+// An object (context, batch, mesh, texture) on a device; the first member of
+// its struct, so that it is destroyed after the buffers.
+struct Live {
+    int device = -1;
+    Live() = default;
+    Live(const Live&) = delete;
+    Live& operator=(const Live&) = delete;
+    void on(int dev);
+    ~Live();
+};
 // A stream of the device for one call (kept for later calls, at most eight)
 // and its return. free_stream: the stream on which memory outliving its call
 // is freed, once nothing uses it any more.
@@ -230,6 +246,7 @@ int dev_limits(int device, const DevLimits** out);
 }  // namespace fgc
 
 struct fgc_texture {
+    fgc::Live live;
     int device = 0;
     int32_t w = 0, h = 0;
     fgc::DevBuf<ushort4> texels;
@@ -237,6 +254,7 @@ struct fgc_texture {
 };
 
 struct fgc_mesh {
+    fgc::Live live;
     int device = 0;
     uint64_t ntri = 0, nline = 0, nuniq = 0;
     fgc::MeshBuf<double> ux, uy, uz;
@@ -419,6 +437,7 @@ int ensure_debug(fgc_context* c);
 }  // namespace fgc
 
 struct fgc_context {
+    fgc::Live live;
     int device = 0;
     int sms = 1;
     cudaStream_t stream = nullptr;      // the stream work is issued on

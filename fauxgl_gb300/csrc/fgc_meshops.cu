@@ -561,6 +561,7 @@ int line_mesh(Work& W, const double* lines, uint64_t n, fgc_mesh** out) {
     fgc_mesh* m = new (std::nothrow) fgc_mesh();
     if (!m) return fail(FGC_ERR_OUT_OF_MEMORY, "host allocation failed");
     m->device = W.dev;
+    m->live.on(W.dev);
     m->ntri = 0;
     m->nline = n;
     int rc = n ? mesh_weld_attrs(m, W.s, W.sms, lines, nullptr, 2 * n) : FGC_OK;
@@ -668,6 +669,7 @@ int fgc_mesh_load_stl(const void* data, uint64_t nbytes, fgc_mesh** out) {
     fgc_mesh* m = new (std::nothrow) fgc_mesh();
     if (!m) return fail(FGC_ERR_OUT_OF_MEMORY, "host allocation failed");
     m->device = dev;
+    m->live.on(dev);
     m->ntri = T;
     m->nline = 0;
     const int rc = T ? mesh_weld_attrs(m, W.s, W.sms, cp.p, nrm.p, 3 * T) : FGC_OK;

@@ -155,6 +155,14 @@ int fgc_clear_color(fgc_context* ctx, const double rgba[4]);
 int fgc_clear_depth(fgc_context* ctx, double value);
 
 /* ---- resources ---------------------------------------------------------- */
+/* Device memory of contexts, batches, meshes, textures and the temporaries of
+ * mesh calls comes from pools of the library, which keep up to 1 GiB each
+ * (three per device) of what has been released for later calls. When the last
+ * object on a device is released they go back to 128 MiB each. fgc_trim_memory
+ * gives everything unused on the current device back to the driver, for a
+ * caller that shares the GPU with another allocator; the next calls that
+ * allocate take longer. Calls of any thread may run meanwhile. */
+int fgc_trim_memory(void);
 /* Upload a triangle soup plus a line list as a device-resident mesh.
  *   tri_pos  ntri*9   V1.Position xyz, V2.Position xyz, V3.Position xyz
  *   tri_nrm  ntri*9   normals, same layout, or NULL (all zero)
