@@ -56,8 +56,8 @@ int enqueue_reads(fgc_batch* b, uint32_t lo, uint32_t hi, cudaStream_t s) {
     const DevLimits* D = nullptr;
     int rc = dev_limits(b->device, &D);
     if (rc) return rc;
-    // every downsample before the first copy: a copy to pageable memory holds
-    // this thread, and a raster kernel that has begun leaves them no room
+    // the range's downsamples before its first copy: a copy to pageable memory
+    // holds this thread, and a raster kernel that has begun leaves them no room
     for (const fgc_batch::ReadBack& r : b->reads) {
         if (r.item < lo || r.item >= hi || r.scale <= 1) continue;
         const fgc_context* c = r.ctx;
@@ -476,11 +476,11 @@ int fgc_batch_autotune(fgc_batch* b, const fgc_batch_item* items, uint64_t n, in
         *ms = t[t.size() / 2];
         return FGC_OK;
     };
-    // coordinate descent over the four shapes, one sweep in this order
+    // coordinate descent over the three shapes, one sweep in this order (`window`
+    // shapes nothing any more: it stays as it was set)
     const int64_t bands[] = {2048, 4096, 8192};
     const int64_t blocks[] = {2048, 4096, 8192, 16384};
     const int frags[] = {512, 768, 1024};
-    const int windows[] = {4, 8, 16, 32};
     PassTuning cur = b->tuning;
     double cur_ms = 0;
     int rc = measure(&cur_ms);
@@ -517,12 +517,6 @@ int fgc_batch_autotune(fgc_batch* b, const fgc_batch_item* items, uint64_t n, in
         if (v == cur.frag_cap) continue;
         PassTuning c = cur;
         c.frag_cap = v;
-        if ((rc = try_one(c))) return rc;
-    }
-    for (int v : windows) {
-        if (v == cur.window) continue;
-        PassTuning c = cur;
-        c.window = v;
         if ((rc = try_one(c))) return rc;
     }
     b->tuning = cur;
