@@ -76,6 +76,7 @@ struct PassPlan {
     int per_max = 1;
     bool any_tri = false, any_line = false, debug_shaded = false;
     int32_t Lmax = 1, band_rows = 1, Rmax = 1;
+    int64_t Lset = 1;            // pixels of the largest band that the tuning asks for
     int precision = FGC_PRECISION_PLAIN;
     RasterFit fit = {0, kSpanUnitsMin, kRasterHeadsMax, kChunkRounds, 0};
     int bsize = 4;               // bytes of a fragment's barycentric (8: some draw is shaded in FP64 throughout)
@@ -127,7 +128,7 @@ int fit_fragments(const DevLimits& D, const PassTuning& T, PassPlan& P) {
     const int stat = D.raster_static[P.precision == FGC_PRECISION_MIXED ? 1 : 0];
     const long two_cta = (long)D.smem_per_sm / 2 - D.smem_reserved_per_block - stat;
     const long one_cta = (long)D.smem_per_block_optin - stat;
-    if (!fit_raster(two_cta, one_cta, T.frag_cap, P.Lmax, P.bsize, P.row_table, P.fit))
+    if (!fit_raster(two_cta, one_cta, T.frag_cap, P.Lmax, P.Lset, P.bsize, P.row_table, P.fit))
         return fail(FGC_ERR_UNSUPPORTED, "frame too wide for the band rasteriser");
     return FGC_OK;
 }
@@ -176,10 +177,13 @@ int plan_pass(const Submission& sub, const std::vector<uint32_t>& idx, const Dev
         v.W = c->W;
         v.H = c->H;
         v.N = c->N;
-        int64_t R = std::max<int64_t>(1, band_pixels / c->W);
-        R = std::min<int64_t>(R, kBandRowsMax);
-        R = std::min<int64_t>(R, c->H);
-        if (R * c->W > 65535) return fail(FGC_ERR_UNSUPPORTED, "frame width above 65535 pixels is not supported");
+        const auto band_rows = [&](int64_t pixels) {
+            return std::min<int64_t>(std::min<int64_t>(std::max<int64_t>(1, pixels / c->W), kBandRowsMax), c->H);
+        };
+        const int64_t R = band_rows(band_pixels);
+        // a band size that was set too large is refused whatever the pass makes of it
+        P.Lset = std::max(P.Lset, band_rows(T.band_pixels) * c->W);
+        if (P.Lset > 65535) return fail(FGC_ERR_UNSUPPORTED, "frame width above 65535 pixels is not supported");
         v.R = (int32_t)R;
         v.L = (int32_t)(R * c->W);
         v.nbands = (uint32_t)ceil_div((uint64_t)c->H, (uint64_t)R);

@@ -110,9 +110,11 @@ struct RasterFit {
 };
 
 // The raster kernel's buffers for bands of up to L pixels within two_cta bytes
-// (two CTAs per SM) or else one_cta. large: the pass's primitives cover several
-// pixels and have row starts. False when the frame is too wide.
-inline bool fit_raster(long two_cta, long one_cta, int frag_cap, int64_t L, int bsize, bool large, RasterFit& f) {
+// (two CTAs per SM) or else one_cta. Lset: the band that the caller's tuning asks
+// for, at least L. large: the pass's primitives cover several pixels and have row
+// starts. False when the frame, or the tuning's band, is too wide.
+inline bool fit_raster(long two_cta, long one_cta, int frag_cap, int64_t L, int64_t Lset, int bsize, bool large,
+                       RasterFit& f) {
     const auto size = [&] { f.smem = raster_smem_bytes(L, f.F, f.su, f.heads, bsize, f.rounds); };
     // primitives of several pixels fill a larger buffer in one round of units
     // (kRowTablePixelsPerElement); small ones do not, and its memory is then
@@ -152,7 +154,7 @@ inline bool fit_raster(long two_cta, long one_cta, int frag_cap, int64_t L, int 
         f.F = smallest_buffer(frag_cap) & ~7;
         size();
     }
-    return L * 8 + smallest_buffer(frag_cap) * 51 <= kBandBytesMax && (long)f.smem <= one_cta;
+    return Lset * 8 + smallest_buffer(frag_cap) * 51 <= kBandBytesMax && (long)f.smem <= one_cta;
 }
 
 }  // namespace fgc

@@ -23,7 +23,7 @@ int main() {
                 for (int bsize : {4, 8})
                     for (bool large : {false, true}) {
                         RasterFit f;
-                        const bool fits = fit_raster(per_sm / 2 - reserved - stat, optin - stat, cap, L, bsize, large, f);
+                        const bool fits = fit_raster(per_sm / 2 - reserved - stat, optin - stat, cap, L, L, bsize, large, f);
                         int least = cap < 4096 ? cap : 4096;
                         while (least > 512) least -= 128;
                         while (least > 256) least /= 2;

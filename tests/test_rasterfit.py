@@ -89,3 +89,33 @@ def test_widest_frame_of_a_cap(gpu_lib, cap, widest):
         assert tuple(batch.Render()[0]) == ref.draw(mesh, ctx.state(), ctx.shader_struct())
         assert np.array_equal(ctx.Image(), ref.color())
         assert np.array_equal(ctx.DepthBuffer.view(np.uint64), ref.depth().view(np.uint64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h,band,accepted", [(320, 180, 26027, True), (320, 180, 26240, False), (320, 180, 31000, False),
+                                               (320, 80, 60000, True), (160, 200, 60000, True), (700, 100, 66000, False)])
+def test_band_size_of_the_tuning(gpu_lib, w, h, band, accepted):
+    """A band of band_pixels (whole rows, at most 128) has to fit, though small passes take smaller ones."""
+    from fauxgl_gb300 import scenes
+    from fauxgl_gb300._abi import FauxGLError
+    from fauxgl_gb300.batch import Batch
+    from fauxgl_gb300.context import NewContext
+    from fauxgl_gb300.mesh import Mesh
+    from fauxgl_gb300.shader import NewPhongShader
+    from fauxgl_gb300.shapes import sphere_positions
+
+    pos = sphere_positions(2)
+    ctx = NewContext(w, h)
+    ctx.Shader = NewPhongShader(scenes.camera_matrix(w, h), scenes.LIGHT, scenes.EYE)
+    batch = Batch()
+    batch.SetTuning(band_pixels=band)
+    batch.Add(ctx, Mesh(pos, pos))
+    if not accepted:
+        with pytest.raises(FauxGLError):
+            batch.Render()
+        return
+    total = batch.Render()[0].TotalPixels
+    alone = NewContext(w, h)
+    alone.Shader = ctx.Shader
+    assert alone.DrawMesh(Mesh(pos, pos)).TotalPixels == total > 0
+    assert np.array_equal(alone.Image(), ctx.Image())
