@@ -144,7 +144,7 @@ struct GeomParams {
     ClipEntry* lclip_list;      // clipped lines (capacity: all lines of the pass)
     uint32_t* lclip_count;
     PoolVertex* pool;           // 21 per clip_list entry
-    PoolVertex32* pool32;       // FP32 copies (draws in the mixed form)
+    PoolVertex32* pool32;       // FP32 copies (draws in the mixed form, certified plain draws)
     ClipPoly* cpoly;            // per clip_list entry
     ClipVert* cvert;            // kClipPoly per clip_list entry
     unsigned long long* prim_total;

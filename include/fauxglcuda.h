@@ -331,10 +331,13 @@ typedef struct fgc_batch_item {
 /* Shapes of the batched pipeline. Results never depend on them;
  * fgc_batch_autotune picks them by measurement. */
 typedef struct fgc_batch_tuning {
-    int32_t band_pixels;          /* raster band size in pixels, whole rows (default 4096) */
-    int32_t prims_per_bin_block;  /* primitives per binning block (default 4096)           */
-    int32_t fragment_cap;         /* fragment buffer of a raster CTA (default 1024; twice
-                                     that for passes of large primitives)                */
+    int32_t band_pixels;          /* raster band size in pixels, whole rows (default 4096);
+                                     small passes take less                              */
+    int32_t prims_per_bin_block;  /* primitives per binning block (default 4096); small
+                                     passes take less                                    */
+    int32_t fragment_cap;         /* fragment buffer of a raster CTA, 256 or more (default
+                                     1024); twice that for passes of large primitives, at
+                                     most 4096, rounded down to a multiple of 8          */
     int32_t use_graph;            /* 1: issue each submission as a CUDA graph              */
     int32_t window;               /* 0-256; kept and reported, the raster stage sizes its
                                      runs over wide triangles itself (default 8)         */

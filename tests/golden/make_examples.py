@@ -7,7 +7,7 @@ RasterizeInfo and the sha256 digests of colour, depth and winner ids to
 tests/golden/examples.json. The digests pin the oracle across machines (the
 GPU test re-renders the oracle where it runs and checks both against them).
 
-    python tests/golden/make_examples.py [reference tree, default /root/reference]
+    python tests/golden/make_examples.py REFERENCE_TREE
 """
 import gzip
 import json
@@ -20,7 +20,9 @@ sys.path.insert(0, ROOT)
 
 
 def main():
-    ref_root = sys.argv[1] if len(sys.argv) > 1 else "/root/reference"
+    if len(sys.argv) != 2:
+        sys.exit("usage: make_examples.py REFERENCE_TREE")
+    ref_root = sys.argv[1]
     from tests import example_scenes as E
     os.makedirs(E.EXAMPLES, exist_ok=True)
     for stl in ("bowser", "hello", "sphere", "cube"):
